@@ -832,14 +832,12 @@ int bqcdg_release_scratch(bqcdg_ctx* c, int what) {
     B.cap = 0;
   }
   if (what & BQCDG_SCRATCH_HMC) {
-    for (double** p : {&c->pgen, &c->mom, &c->mom_old}) {
+    for (double** p : {&c->pgen, &c->mom, &c->mom_old, &c->wbuf}) {
       c->release(*p);
       *p = nullptr;
     }
-    for (double2** p : {&c->wbuf, &c->gauge_bck}) {
-      c->release(*p);
-      *p = nullptr;
-    }
+    c->release(c->gauge_bck);
+    c->gauge_bck = nullptr;
   }
   return BQCDG_OK;
 }
@@ -1239,7 +1237,7 @@ int bqcdg_quda_solver(bqcdg_ctx* c, double* x, const double* b, const bqcdg_para
 namespace bqcdg_host {
 int ensure_force_bufs(bqcdg_ctx* c) {
   if (!c->pgen) CK(c->alloc((void**)&c->pgen, (size_t)64 * c->g.volh * sizeof(double)));
-  if (!c->wbuf) CK(c->alloc((void**)&c->wbuf, (size_t)54 * c->g.stride * sizeof(double2)));
+  if (!c->wbuf) CK(c->alloc((void**)&c->wbuf, 2 * clover_w_field(c->g) * sizeof(double)));
   return BQCDG_OK;
 }
 }  // namespace bqcdg_host
@@ -1297,13 +1295,9 @@ int dsf_core(bqcdg_ctx* c, double* p, double step, const bqcdg_params* par, doub
   double s1 = -step * 2.0 * (par->csw_kappa / 8.0);
   double s2 = -step * 2.0 * (par->csw_kappa / 8.0) * par->kappa * par->kappa;
   if (s1 != 0.0) {
-    launch_clover_bsa(c->g, c->wbuf, db, da, c->stream);
-    launch_clover_d(c->g, p, c->gauge64, c->wbuf, 0, s1, c->stream);
-    CKL();
-  }
-  if (s2 != 0.0) {
-    launch_clover_bsa(c->g, c->wbuf, dbt, dat, c->stream);
-    launch_clover_d(c->g, p, c->gauge64, c->wbuf, 1, s2, c->stream);
+    launch_clover_bsa(c->g, c->wbuf, db, da, s1, c->stream);
+    if (s2 != 0.0) launch_clover_bsa(c->g, c->wbuf + clover_w_field(c->g), dbt, dat, s2, c->stream);
+    launch_clover_d(c->g, p, c->gauge64, c->wbuf, s2 != 0.0 ? 2 : 0, c->stream);
     CKL();
   }
   return BQCDG_OK;
@@ -1342,8 +1336,8 @@ int bqcdg_clover_dsf(bqcdg_ctx* c, int eo, double* p, const double* b, const dou
   CK(cudaMemcpyAsync(c->pgen, p, pn, cudaMemcpyHostToDevice, c->stream));
   if ((st = upload_spinor(c, a, da))) return st;
   if ((st = upload_spinor(c, b, db))) return st;
-  launch_clover_bsa(c->g, c->wbuf, db, da, c->stream);
-  launch_clover_d(c->g, c->pgen, c->gauge64, c->wbuf, eo, s, c->stream);
+  launch_clover_bsa(c->g, c->wbuf, db, da, s, c->stream);
+  launch_clover_d(c->g, c->pgen, c->gauge64, c->wbuf, eo, c->stream);
   CKL();
   CK(cudaMemcpyAsync(p, c->pgen, pn, cudaMemcpyDeviceToHost, c->stream));
   CK(cudaStreamSynchronize(c->stream));
@@ -1357,8 +1351,8 @@ namespace bqcdg_host {
 int dsd_core(bqcdg_ctx* c, double* p, int eo, double s) {
   // the fields hold T (bqcdg_clover_init_t), not BQCD's blocks
   if (c && c->g.clover_t) return BQCDG_EUNSUPPORTED;
-  launch_clover_ts(c->g, c->wbuf, c->Ainv[eo], c->stream);
-  launch_clover_d(c->g, p, c->gauge64, c->wbuf, eo, s, c->stream);
+  launch_clover_ts(c->g, c->wbuf, c->Ainv[eo], s, c->stream);
+  launch_clover_d(c->g, p, c->gauge64, c->wbuf, eo, c->stream);
   CKL();
   return BQCDG_OK;
 }

@@ -199,13 +199,17 @@ void launch_gauge_check(const Geom& g, const double2* gauge, RedScratch red, dou
 // hopping force (dsf.F90:75-100): p(eo,mu) from a,b (even) and at,bt (odd)
 void launch_dsf_hop(const Geom& g, double* p, const double2* gauge, const double2* a, const double2* b,
                     const double2* at, const double2* bt, double s, cudaStream_t st);
-// w planes of clover_bsa (6 planes x 9 complex per site) -> wbuf [6][9][stride]
-void launch_clover_bsa(const Geom& g, double2* w, const double2* b, const double2* a, cudaStream_t st);
-// w planes of clover_ts from the halved inverse blocks (clover_t_init + ts)
-void launch_clover_ts(const Geom& g, double2* w, const double2* ainv, cudaStream_t st);
-// clover_d: p(link) += contributions of the w planes of parity eo_w
-void launch_clover_d(const Geom& g, double* p, const double2* gauge, const double2* w, int eo_w, double s,
-                     cudaStream_t st);
+// The sigma_mu_nu planes w of one parity as s (w + w^+), 9 reals per plane and
+// site (force.cu): clover_w_field(g) doubles per parity
+inline size_t clover_w_field(const Geom& g) { return (size_t)54 * g.stride; }
+// of clover_bsa, from the spinors b, a of that parity
+void launch_clover_bsa(const Geom& g, double* w, const double2* b, const double2* a, double s, cudaStream_t st);
+// of clover_ts, from the halved inverse blocks (clover_t_init + ts)
+void launch_clover_ts(const Geom& g, double* w, const double2* ainv, double s, cudaStream_t st);
+// clover_d: p(link) += contributions of the planes w of parity eo_w, or, with
+// eo_w = 2, of both parities (w the even field, the odd one after it) in one
+// pass over the links
+void launch_clover_d(const Geom& g, double* p, const double2* gauge, const double* w, int eo_w, cudaStream_t st);
 
 // ---- clover construction (clover_init.cu) ----
 // clover_init.F90 + clover_inv.F90 on device: A, Ainv, B of each parity whose

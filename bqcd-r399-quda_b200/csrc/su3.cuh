@@ -141,4 +141,84 @@ __device__ __forceinline__ void staple(const Geom& g, const double2* gauge, cons
   }
 }
 
+// ---------------------------------------------------------------------------
+// products with links that stay in memory, for kernels of one thread per link
+// ---------------------------------------------------------------------------
+// element (r, c) of op(U) of a link in memory (columns of 3)
+template <bool DAG>
+__device__ __forceinline__ C64 mel(const double2* u, int stride, int r, int c) {
+  const double2 t = __ldg(u + (DAG ? r * 3 + c : c * 3 + r) * stride);
+  return DAG ? mkc(t.x, -t.y) : mkc(t.x, t.y);
+}
+__device__ __forceinline__ C64 dmul(double a, C64 b) { return mkc(a * b.x, a * b.y); }
+__device__ __forceinline__ C64 dfma(C64 acc, double a, C64 b) { return mkc(fma(a, b.x, acc.x), fma(a, b.y, acc.y)); }
+
+// the row r of op(U) times m is added to (or stored in) t[r][.]; U's row is
+// loaded where it is used, so only m and t are live
+template <bool DAG, bool ADD>
+__device__ __forceinline__ void lmul(L64& t, const double2* u, int stride, const L64& m) {
+#pragma unroll
+  for (int r = 0; r < 3; r++) {
+    const C64 a0 = mel<DAG>(u, stride, r, 0), a1 = mel<DAG>(u, stride, r, 1), a2 = mel<DAG>(u, stride, r, 2);
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+      C64 x = ADD ? fma_c(t.m[r][c], a0, m.m[0][c]) : a0 * m.m[0][c];
+      x = fma_c(x, a1, m.m[1][c]);
+      t.m[r][c] = fma_c(x, a2, m.m[2][c]);
+    }
+  }
+}
+// t += m op(U), column by column of op(U)
+template <bool DAG>
+__device__ __forceinline__ void rmul_add(L64& t, const L64& m, const double2* u, int stride) {
+#pragma unroll
+  for (int c = 0; c < 3; c++) {
+    const C64 a0 = mel<DAG>(u, stride, 0, c), a1 = mel<DAG>(u, stride, 1, c), a2 = mel<DAG>(u, stride, 2, c);
+#pragma unroll
+    for (int r = 0; r < 3; r++) {
+      C64 x = fma_c(t.m[r][c], m.m[r][0], a0);
+      x = fma_c(x, m.m[r][1], a1);
+      t.m[r][c] = fma_c(x, m.m[r][2], a2);
+    }
+  }
+}
+// m = op(U)
+template <bool DAG>
+__device__ __forceinline__ void lload(L64& m, const double2* u, int stride) {
+#pragma unroll
+  for (int r = 0; r < 3; r++)
+#pragma unroll
+    for (int c = 0; c < 3; c++) m.m[r][c] = mel<DAG>(u, stride, r, c);
+}
+
+// the row (y, z, t) shifts by +-1 in a direction (x is shifted by its
+// coordinate); shifts in different directions add
+struct Shifts {
+  int f[4], b[4];    // row shifts, 0 for x
+  int xf, xb, xh;    // half coordinates of x + 1, x - 1, x
+  int base;
+};
+__device__ __forceinline__ Shifts make_shifts(const Geom& g, const Site& st) {
+  Shifts q;
+  int step = g.Lxh;
+  q.f[0] = q.b[0] = 0;
+#pragma unroll
+  for (int d = 1; d < 4; d++) {
+    q.f[d] = st.x[d] == g.L[d] - 1 ? -(g.L[d] - 1) * step : step;
+    q.b[d] = st.x[d] == 0 ? (g.L[d] - 1) * step : -step;
+    step *= g.L[d];
+  }
+  q.xf = (st.x[0] == g.L[0] - 1 ? 0 : st.x[0] + 1) >> 1;
+  q.xb = (st.x[0] == 0 ? g.L[0] - 1 : st.x[0] - 1) >> 1;
+  q.xh = st.x[0] >> 1;
+  q.base = st.base;
+  return q;
+}
+// entry k, known at run time, without indexing (an indexed array goes to
+// local memory)
+__device__ __forceinline__ int pick4(int a0, int a1, int a2, int a3, int k) {
+  return k < 2 ? (k == 0 ? a0 : a1) : (k == 2 ? a2 : a3);
+}
+__device__ __forceinline__ int pick(const int a[4], int k) { return pick4(a[0], a[1], a[2], a[3], k); }
+
 }  // namespace bqcdg
