@@ -167,29 +167,51 @@ void launch_hmc_u(const Geom& g, double2* gauge, const double* p, double step, c
 }
 
 // dsg.F90:28-53: p(link) += s Im Tr(lambda_j U S), S the sum of the six
-// staples of the link, s = -step beta / 3 (the staple sum reads links only,
-// so every link is independent)
-__global__ void __launch_bounds__(kBlock) k_dsg(Geom g, const double2* gauge, double* p, double s) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  const int me = blockIdx.y;
+// staples of the link (staple.F90:28-63), s = -step beta / 3 (the staple sum
+// reads links only, so every link is independent).  The six staples are two
+// per plane with the links' rows read where they are used and a plane loop
+// that is not unrolled, and the 8 links of a site block are neighbouring CTAs:
+// 0.45 ms at 24^3x48, against 1.12 ms with every matrix in registers (194, 2
+// CTAs per SM) and the link classes in sequence.  13 products per link are
+// 0.20 ms of FP64; the rest is the latency of 19 link reads per link.
+__global__ void __launch_bounds__(kBlock, 3) k_dsg(Geom g, const double2* gauge, double* p, double s) {
+  const int i = (blockIdx.x >> 3) * blockDim.x + threadIdx.x;
+  const int me = blockIdx.x & 7;
   if (i >= g.volh) return;
-  const int mu = me >> 1, eo = me & 1;
-  const Site st = site_coords(g, i, eo);
-  L64 uuu, u, w;
-  staple(g, gauge, st.x, mu, uuu);
-  GaugeView<Prec::F64>{(double2*)gauge, g.stride}.load(mu, eo, i, u);
-  mul2(w, u, false, uuu, false);
+  const int mu = me >> 1, e = me & 1, S = g.stride;
+  const Shifts q = make_shifts(g, site_coords(g, i, e));
+  const int fmu = pick(q.f, mu), xmu = mu == 0 ? q.xf : q.xh;
+  const int id = q.base + fmu + xmu;  // x + mu
+  L64 X, m, k;
+  lzero(X);
+#pragma unroll 1
+  for (int nu = 0; nu < 4; nu++) {
+    if (nu == mu) continue;
+    const int fn = pick(q.f, nu), bn = pick(q.b, nu);
+    const int ie = q.base + fn + (nu == 0 ? q.xf : q.xh), jf = q.base + bn + (nu == 0 ? q.xb : q.xh);
+    const int ic = q.base + fmu + bn + (nu == 0 ? q.xb : xmu);
+    const double2 *Um_o = gauge + (size_t)((mu * 2 + 1 - e) * 9) * S, *Un_o = gauge + (size_t)((nu * 2 + 1 - e) * 9) * S,
+                  *Un_e = gauge + (size_t)((nu * 2 + e) * 9) * S;
+    lload<true>(m, Un_e + i, S);  // U_nu(x+mu) U_mu(x+nu)^+ U_nu(x)^+
+    lmul<true, false>(k, Um_o + ie, S, m);
+    lmul<false, true>(X, Un_o + id, S, k);
+    lload<false>(m, Un_o + jf, S);  // U_nu(x-nu+mu)^+ U_mu(x-nu)^+ U_nu(x-nu)
+    lmul<true, false>(k, Um_o + jf, S, m);
+    lmul<true, true>(X, Un_e + ic, S, k);
+  }
+  lmul<false, false>(m, gauge + (size_t)(me * 9) * S + i, S, X);
   double* pp = mom_of(p, g, me, i);
-  double q[8];
+  double a[8];
 #pragma unroll
-  for (int j = 0; j < 8; j++) q[j] = pp[j];
-  im_tr_j(q, w, s);
+  for (int j = 0; j < 8; j++) a[j] = pp[j];
+  im_tr_j(a, m, s);
 #pragma unroll
-  for (int j = 0; j < 8; j++) pp[j] = q[j];
+  for (int j = 0; j < 8; j++) pp[j] = a[j];
 }
 
 void launch_dsg(const Geom& g, const double2* gauge, double* p, double s, cudaStream_t st) {
-  k_dsg<<<dim3(nblocks(g.volh), 8), kBlock, 0, st>>>(g, gauge, p, s);
+  const int nb = 8 * nblocks(g.volh);
+  k_dsg<<<nb, kBlock, 0, st>>>(g, gauge, p, s);
 }
 
 // sum over all 64 volh momentum entries of (a - b)^2 (b = nullptr: a^2);
