@@ -890,7 +890,7 @@ static int clover_init_t(bqcdg_ctx* c, double csw) {
   const size_t n = (size_t)36 * c->g.stride * sizeof(double2);
   if (!c->A[0]) CK(c->alloc((void**)&c->A[0], n));
   if (!c->Ainv[1]) CK(c->alloc((void**)&c->Ainv[1], n));
-  if (!c->clov_tmp) CK(c->alloc((void**)&c->clov_tmp, (size_t)54 * clover_init_chunk(c->g) * sizeof(double2)));
+  if (!c->clov_tmp) CK(c->alloc((void**)&c->clov_tmp, clover_init_tmp(c->g) * sizeof(double2)));
   double2* t[2] = {c->A[0], c->Ainv[1]};
   launch_clover_t(c->g, c->gauge64, csw, t, c->clov_tmp, c->stream);
   CKL();
@@ -995,7 +995,7 @@ int bqcdg_clover_init(bqcdg_ctx* c, double csw_kappa) {
     if (!c->Ainv[eo]) CK(c->alloc((void**)&c->Ainv[eo], n));
     if (!c->B[eo]) CK(c->alloc((void**)&c->B[eo], n));
   }
-  if (!c->clov_tmp) CK(c->alloc((void**)&c->clov_tmp, (size_t)54 * clover_init_chunk(c->g) * sizeof(double2)));
+  if (!c->clov_tmp) CK(c->alloc((void**)&c->clov_tmp, clover_init_tmp(c->g) * sizeof(double2)));
   launch_clover_init(c->g, c->gauge64, csw_kappa, c->A, c->Ainv, c->B, c->clov_tmp, c->stream);
   CKL();
   CK(cudaStreamSynchronize(c->stream));
@@ -1022,7 +1022,7 @@ int bqcdg_clover_init_solver(bqcdg_ctx* c, double csw_kappa) {
   double2* a[2] = {c->A[0], nullptr};
   double2* ai[2] = {nullptr, c->Ainv[1]};
   double2* b[2] = {nullptr, nullptr};
-  if (!c->clov_tmp) CK(c->alloc((void**)&c->clov_tmp, (size_t)54 * clover_init_chunk(c->g) * sizeof(double2)));
+  if (!c->clov_tmp) CK(c->alloc((void**)&c->clov_tmp, clover_init_tmp(c->g) * sizeof(double2)));
   launch_clover_init(c->g, c->gauge64, csw_kappa, a, ai, b, c->clov_tmp, c->stream);
   CKL();
   CK(cudaStreamSynchronize(c->stream));

@@ -214,8 +214,10 @@ void launch_clover_d(const Geom& g, double* p, const double2* gauge, const doubl
 // ---- clover construction (clover_init.cu) ----
 // clover_init.F90 + clover_inv.F90 on device: A, Ainv, B of each parity whose
 // pointers are given (null: not computed), in chunks of clover_init_chunk(g)
-// sites through tmp (54 complex per chunk site: the six field strengths)
+// sites through tmp (clover_init_tmp(g) complex: the six field strengths of a
+// chunk, 5 complex each)
 int clover_init_chunk(const Geom& g);
+inline size_t clover_init_tmp(const Geom& g) { return (size_t)30 * clover_init_chunk(g); }
 void launch_clover_init(const Geom& g, const double2* gauge, double csw_kappa, double2* a[2], double2* ainv[2],
                         double2* b[2], double2* tmp, cudaStream_t s);
 // T = (-c_sw / 8)(p +- q) of each chiral block, packed like A, for the

@@ -30,33 +30,6 @@ __device__ __forceinline__ void mul2(L64& r, const L64& a, bool da, const L64& b
       r.m[i][j] = t;
     }
 }
-// r = op(a) op(b) op(c)
-__device__ __forceinline__ void mul3(L64& r, const L64& a, bool da, const L64& b, bool db, const L64& c, bool dc) {
-  L64 t;
-  mul2(t, a, da, b, db);
-  mul2(r, t, false, c, dc);
-}
-// r = op(a) op(b) op(c), one row of op(a) op(b) at a time: the same
-// products and sums as mul3, with a 3-element temporary instead of a matrix
-__device__ __forceinline__ void mul3_rows(L64& r, const L64& a, bool da, const L64& b, bool db, const L64& c,
-                                          bool dc) {
-#pragma unroll
-  for (int i = 0; i < 3; i++) {
-    C64 t[3];
-#pragma unroll
-    for (int k = 0; k < 3; k++) {
-      C64 x = el(a, i, 0, da) * el(b, 0, k, db);
-      x = x + el(a, i, 1, da) * el(b, 1, k, db);
-      t[k] = x + el(a, i, 2, da) * el(b, 2, k, db);
-    }
-#pragma unroll
-    for (int j = 0; j < 3; j++) {
-      C64 x = t[0] * el(c, 0, j, dc);
-      x = x + t[1] * el(c, 1, j, dc);
-      r.m[i][j] = x + t[2] * el(c, 2, j, dc);
-    }
-  }
-}
 // su3.F90:196-214: p_j += s Im Tr(lambda_j v)
 __device__ __forceinline__ void im_tr_j(double p[8], const L64& v, double s) {
   p[0] += s * (v.m[0][1].y + v.m[1][0].y);
@@ -189,6 +162,31 @@ __device__ __forceinline__ void lload(L64& m, const double2* u, int stride) {
   for (int r = 0; r < 3; r++)
 #pragma unroll
     for (int c = 0; c < 3; c++) m.m[r][c] = mel<DAG>(u, stride, r, c);
+}
+
+// the same with a run-time dagger
+__device__ __forceinline__ C64 mel_rt(const double2* u, int stride, int r, int c, bool dag) {
+  const double2 t = __ldg(u + (dag ? r * 3 + c : c * 3 + r) * stride);
+  return mkc(t.x, dag ? -t.y : t.y);
+}
+__device__ __forceinline__ void lload_rt(L64& m, const double2* u, int stride, bool dag) {
+#pragma unroll
+  for (int r = 0; r < 3; r++)
+#pragma unroll
+    for (int c = 0; c < 3; c++) m.m[r][c] = mel_rt(u, stride, r, c, dag);
+}
+template <bool ADD>
+__device__ __forceinline__ void lmul_rt(L64& t, const double2* u, int stride, bool dag, const L64& m) {
+#pragma unroll
+  for (int r = 0; r < 3; r++) {
+    const C64 a0 = mel_rt(u, stride, r, 0, dag), a1 = mel_rt(u, stride, r, 1, dag), a2 = mel_rt(u, stride, r, 2, dag);
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+      C64 x = ADD ? fma_c(t.m[r][c], a0, m.m[0][c]) : a0 * m.m[0][c];
+      x = fma_c(x, a1, m.m[1][c]);
+      t.m[r][c] = fma_c(x, a2, m.m[2][c]);
+    }
+  }
 }
 
 // the row (y, z, t) shifts by +-1 in a direction (x is shifted by its
