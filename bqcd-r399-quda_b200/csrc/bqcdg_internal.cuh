@@ -184,8 +184,61 @@ __host__ __device__ __forceinline__ int hop_sign(const Geom& g, const Site& s, i
 }
 
 // ---------------------------------------------------------------------------
+// chained launches (launch_chain): the CTAs of a launch may start while the
+// kernel before it in the stream drains.  chain_wait() returns once that
+// kernel has finished and its writes are visible, and only then lets the next
+// kernel's CTAs start.  Every thread of every kernel launched this way calls
+// it before it leaves, so kernels finish in stream order, and before it,
+// a kernel reads only what was written two or more launches earlier and
+// writes nothing.  (In a kernel launched the ordinary way it returns at once.)
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ void chain_wait() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+// p, as known only after the chain_wait before: no load through it can be
+// moved ahead of the wait
+template <typename T>
+__device__ __forceinline__ T* after_wait(T* p) {
+  asm volatile("" : "+l"(p)::"memory");
+  return p;
+}
+
+// ---------------------------------------------------------------------------
 // field views
 // ---------------------------------------------------------------------------
+// spinor loads: ld.global, not the read-only path (ld.global.nc), since a
+// chained kernel starts before the field it gathers from is written; the
+// compiler may reorder them like read-only loads, and takes those of a field
+// that the launch before writes through a pointer from after_wait.  (As plain
+// C++ loads k_pass2<int16> at 32^3x64 took 111 instead of 104 us.)
+__device__ __forceinline__ double2 ld_field(const double2* p) {
+  double2 r;
+  asm("ld.global.v2.f64 {%0, %1}, [%2];" : "=d"(r.x), "=d"(r.y) : "l"(p));
+  return r;
+}
+__device__ __forceinline__ float4 ld_field(const float4* p) {
+  float4 r;
+  asm("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(r.x), "=f"(r.y), "=f"(r.z), "=f"(r.w) : "l"(p));
+  return r;
+}
+__device__ __forceinline__ int4 ld_field(const int4* p) {
+  int4 r;
+  asm("ld.global.v4.s32 {%0, %1, %2, %3}, [%4];" : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w) : "l"(p));
+  return r;
+}
+__device__ __forceinline__ int2 ld_field(const int2* p) {
+  int2 r;
+  asm("ld.global.v2.s32 {%0, %1}, [%2];" : "=r"(r.x), "=r"(r.y) : "l"(p));
+  return r;
+}
+__device__ __forceinline__ float ld_field(const float* p) {
+  float r;
+  asm("ld.global.f32 %0, [%1];" : "=f"(r) : "l"(p));
+  return r;
+}
+
 template <Prec P>
 struct SpinorView;
 
@@ -199,7 +252,7 @@ struct SpinorView<Prec::F64> {
     for (int c = 0; c < 3; c++)
 #pragma unroll
       for (int sp = 0; sp < 4; sp++) {
-        double2 t = __ldg(v + (c * 4 + sp) * stride + i);
+        double2 t = ld_field(v + (c * 4 + sp) * stride + i);
         s.c[sp][c] = mkc(t.x, t.y);
       }
   }
@@ -209,7 +262,7 @@ struct SpinorView<Prec::F64> {
     for (int c = 0; c < 3; c++)
 #pragma unroll
       for (int k = 0; k < 2; k++) {
-        double2 t = __ldg(v + (c * 4 + s0 + k) * stride + i);
+        double2 t = ld_field(v + (c * 4 + s0 + k) * stride + i);
         h[k][c] = mkc(t.x, t.y);
       }
   }
@@ -245,7 +298,7 @@ struct SpinorView<Prec::F32> {
   __device__ __forceinline__ void load(int i, Spinor<float>& s) const {
 #pragma unroll
     for (int k = 0; k < 6; k++) {
-      float4 t = __ldg(v + k * stride + i);
+      float4 t = ld_field(v + k * stride + i);
       int k0 = 2 * k, k1 = 2 * k + 1;
       s.c[k0 & 3][k0 >> 2] = mkc(t.x, t.y);
       s.c[k1 & 3][k1 >> 2] = mkc(t.z, t.w);
@@ -255,7 +308,7 @@ struct SpinorView<Prec::F32> {
     // components (c*4+s0, c*4+s0+1) sit in float4 number c*2 + s0/2
 #pragma unroll
     for (int c = 0; c < 3; c++) {
-      float4 t = __ldg(v + (c * 2 + (s0 >> 1)) * stride + i);
+      float4 t = ld_field(v + (c * 2 + (s0 >> 1)) * stride + i);
       h[0][c] = mkc(t.x, t.y);
       h[1][c] = mkc(t.z, t.w);
     }
@@ -335,10 +388,10 @@ struct SpinorView<Prec::F16> {
   // applies sc once, after the linear projection and transport).  int4
   // number k holds colour k, spins 0..3, one complex per 32-bit word.
   __device__ __forceinline__ void load_raw(int i, Spinor<float>& s, float& sc) const {
-    sc = __ldg(norm + i) * (1.0f / 32767.0f);
+    sc = ld_field(norm + i) * (1.0f / 32767.0f);
 #pragma unroll
     for (int k = 0; k < 3; k++) {
-      const int4 t = __ldg(v + k * stride + i);
+      const int4 t = ld_field(v + k * stride + i);
       const float2 a = u16x2_to_f2(t.x), b = u16x2_to_f2(t.y), c = u16x2_to_f2(t.z), d = u16x2_to_f2(t.w);
       s.c[0][k] = mkc(a.x, a.y);
       s.c[1][k] = mkc(b.x, b.y);
@@ -348,11 +401,11 @@ struct SpinorView<Prec::F16> {
   }
   // spins s0, s0+1 (s0 even) of every colour: one half of each int4
   __device__ __forceinline__ void load_pair_raw(int i, int s0, cx<float> h[2][3], float& sc) const {
-    sc = __ldg(norm + i) * (1.0f / 32767.0f);
+    sc = ld_field(norm + i) * (1.0f / 32767.0f);
 #pragma unroll
     for (int c = 0; c < 3; c++) {
       const int2* p = reinterpret_cast<const int2*>(v + c * stride + i);
-      const int2 t = __ldg(p + (s0 >> 1));
+      const int2 t = ld_field(p + (s0 >> 1));
       const float2 a = u16x2_to_f2(t.x), b = u16x2_to_f2(t.y);
       h[0][c] = mkc(a.x, a.y);
       h[1][c] = mkc(b.x, b.y);
@@ -361,10 +414,10 @@ struct SpinorView<Prec::F16> {
   // biased values (q + kQBias, see u16x2_biased) of all 12 components,
   // F[spin][colour] = (re, im); the true value is (F - kQBias) * sc
   __device__ __forceinline__ void load_biased(int i, float2 F[4][3], float& sc) const {
-    sc = __ldg(norm + i) * (1.0f / 32767.0f);
+    sc = ld_field(norm + i) * (1.0f / 32767.0f);
 #pragma unroll
     for (int k = 0; k < 3; k++) {
-      const int4 t = __ldg(v + k * stride + i);
+      const int4 t = ld_field(v + k * stride + i);
       F[0][k] = u16x2_biased(t.x);
       F[1][k] = u16x2_biased(t.y);
       F[2][k] = u16x2_biased(t.z);
@@ -394,6 +447,14 @@ struct SpinorView<Prec::F16> {
   }
   __device__ __forceinline__ void store(int i, const Spinor<float>& s) const { store_scaled(i, s, 1.0f); }
 };
+
+// the view through pointers from after_wait
+template <Prec P>
+__device__ __forceinline__ SpinorView<P> after_wait(SpinorView<P> v) {
+  v.v = after_wait(v.v);
+  if constexpr (P == Prec::F16) v.norm = after_wait(v.norm);
+  return v;
+}
 
 // Loads of data that a pass reads once (links, clover blocks): read-only
 // path without L1 allocation, so these streamed fields leave L1 to the
@@ -1033,7 +1094,7 @@ __device__ __forceinline__ void wilson_hop(const Geom& g, int e, int i, const Si
 // bit-identical; it needs about 40 more registers.
 template <bool DAG>
 __device__ __forceinline__ void wilson_hop_lf(const Geom& g, int e, int i, const Site& st,
-                                              const SpinorView<Prec::F16>& in, const GaugeView<Prec::F16>& U,
+                                              const SpinorView<Prec::F16>& in0, const GaugeView<Prec::F16>& U,
                                               Spinor<float>& b, float hscale = 1.f) {
   const int o = 1 - e;
   const uint2* ub = reinterpret_cast<const uint2*>(U.v);
@@ -1050,6 +1111,8 @@ __device__ __forceinline__ void wilson_hop_lf(const Geom& g, int e, int i, const
       W[mu][1][w] = ld_once(ub + (size_t)((mu * 2 + o) * 3 + w) * S + J[mu][1]);
     }
   }
+  chain_wait();  // the links do not depend on the launch before
+  const SpinorView<Prec::F16> in = after_wait(in0);
 #pragma unroll
   for (int mu = 3; mu >= 0; mu--) {
 #pragma unroll
@@ -1106,11 +1169,12 @@ struct Tile {
   int nsb;  // site blocks per RHS
   int i;    // site of this thread
 };
-__device__ __forceinline__ Tile tile(int nr) {
+// the first `extra` site blocks of the launch are for other work: sb < 0
+__device__ __forceinline__ Tile tile(int nr, int extra = 0) {
   Tile t;
   t.rhs = blockIdx.x % nr;
-  t.sb = blockIdx.x / nr;
-  t.nsb = gridDim.x / nr;
+  t.sb = (int)(blockIdx.x / nr) - extra;
+  t.nsb = gridDim.x / nr - extra;
   t.i = t.sb * blockDim.x + threadIdx.x;
   return t;
 }

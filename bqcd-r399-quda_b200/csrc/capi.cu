@@ -94,17 +94,19 @@ int check_op(bqcdg_ctx* c, const bqcdg_params* p) {
 }
 
 // out_e = M~ in_e  (dag: M~^+), with rho for W; t_o scratch (odd)
+// (chain: the launch before is a pass of the same operator)
 void apply_mtil(bqcdg_ctx* c, Prec p, bool dag, SpinorPtr out, SpinorPtr in, SpinorPtr t, const OpParams& op,
-                double* norm_out, CgScalars* cg) {
+                double* norm_out, CgScalars* cg, bool chain) {
   const Geom& g = geom_of(c, p);
-  launch_mtil_pass1(p, g, dag, t, in, gauge_of(c, p), ainv_of(c, p), op, cg, c->stream);
-  launch_mtil_pass2(p, g, dag, out, t, in, gauge_of(c, p), aee_of(c, p), op, c->red, norm_out, cg, c->stream);
+  launch_mtil_pass1(p, g, dag, t, in, gauge_of(c, p), ainv_of(c, p), op, cg, c->stream, 1, nullptr, AlphaFin{}, chain);
+  launch_mtil_pass2(p, g, dag, out, t, in, gauge_of(c, p), aee_of(c, p), op, c->red, norm_out, cg, c->stream, 1,
+                    nullptr, nullptr, false, true);
 }
 
 // out = (W^+ W) in in precision p; scratch t (odd), q (even)
 void apply_mdagm(bqcdg_ctx* c, Prec p, SpinorPtr out, SpinorPtr in, SpinorPtr t, SpinorPtr q, const OpParams& op) {
   apply_mtil(c, p, false, q, in, t, op, nullptr, nullptr);
-  apply_mtil(c, p, true, out, q, t, op, nullptr, nullptr);
+  apply_mtil(c, p, true, out, q, t, op, nullptr, nullptr, true);
 }
 
 int read_cg(bqcdg_ctx* c) {
@@ -246,18 +248,19 @@ int cg_core(bqcdg_ctx* c, double2* x, double2* b, const OpParams& op, Prec slopp
       // they time.
       const bool timed = k == 1;
       if (timed) kt.begin();
-      launch_mtil_pass1(sloppy, gs, false, t, p, gauge_of(c, sloppy), ainv_of(c, sloppy), op, c->dcg, c->stream);
+      launch_mtil_pass1(sloppy, gs, false, t, p, gauge_of(c, sloppy), ainv_of(c, sloppy), op, c->dcg, c->stream, 1,
+                        nullptr, AlphaFin{}, true);
       if (timed) kt.end();
       launch_mtil_pass2(sloppy, gs, false, q, t, p, gauge_of(c, sloppy), aee_of(c, sloppy), op, c->red, nullptr,
-                        c->dcg, c->stream, 1, nullptr, nullptr, true);
+                        c->dcg, c->stream, 1, nullptr, nullptr, true, true);
       if (timed) kt.begin();
       launch_mtil_pass1(sloppy, gs, true, t, q, gauge_of(c, sloppy), ainv_of(c, sloppy), op, c->dcg, c->stream, 1,
-                        nullptr, AlphaFin{c->red.partial, c->red.maxblocks, c->dcg});
+                        nullptr, AlphaFin{c->red.partial, c->red.maxblocks, c->dcg}, true);
       if (timed) kt.end();
-      launch_cg_pass4(sloppy, gs, t, q, gauge_of(c, sloppy), aee_of(c, sloppy), op, p, xs, rs, c->red, c->dcg,
-                      c->stream, 1, false, nullptr, nullptr, true);
+      launch_cg_pass4(sloppy, gs, t, q, gauge_of(c, sloppy), aee_of(c, sloppy), op, rs, c->red, c->dcg, c->stream, 1,
+                      nullptr, nullptr, true, true);
       launch_cg_step(c->red, c->dcg, 1, nblocks(gs.volh), c->stream);
-      launch_cg_pupdate(sloppy, g, p, rs, c->dcg, c->stream, 1, xs, iter0 + k + 1);
+      launch_cg_pupdate(sloppy, g, p, rs, c->dcg, c->stream, 1, xs, CgExpect{{iter0 + k + 1}}, true);
     }
     CKL();
     int st = read_cg(c);
@@ -488,29 +491,32 @@ int cg_batch(bqcdg_ctx* c, double2** x, double2** b, int nb, const OpParams& op,
     return false;
   };
   while (running()) {
+    CgExpect expect{};
+    for (int k = 0; k < nb; k++) expect.n[k] = c->hcg[k].iter;
     for (int it = 0; it < batch; it++) {
+      for (int k = 0; k < nb; k++) expect.n[k]++;
       if (nbt > 1) {
         launch_mtil_pass1_n(sloppy, g, false, B.t, B.p, gauge_of(c, sloppy), ainv_of(c, sloppy), op, c->dcg,
-                            c->stream, nb, nbt);
+                            c->stream, nb, nbt, AlphaFin{}, true);
         launch_mtil_pass2_n(sloppy, g, B.q, B.t, B.p, gauge_of(c, sloppy), aee_of(c, sloppy), op, c->red, c->dcg,
-                            c->stream, nb, drho, nbt, true);
+                            c->stream, nb, drho, nbt, true, true);
         launch_mtil_pass1_n(sloppy, g, true, B.t, B.q, gauge_of(c, sloppy), ainv_of(c, sloppy), op, c->dcg,
-                            c->stream, nb, nbt, AlphaFin{c->red.partial, c->red.maxblocks, c->dcg});
-        launch_cg_pass4_n(sloppy, g, B.t, B.q, gauge_of(c, sloppy), aee_of(c, sloppy), op, B.p, B.xs, B.rs, c->red,
-                          c->dcg, c->stream, nb, drho, nbt, true);
+                            c->stream, nb, nbt, AlphaFin{c->red.partial, c->red.maxblocks, c->dcg}, true);
+        launch_cg_pass4_n(sloppy, g, B.t, B.q, gauge_of(c, sloppy), aee_of(c, sloppy), op, B.rs, c->red, c->dcg,
+                          c->stream, nb, drho, nbt, true, true);
         launch_cg_step(c->red, c->dcg, nb, nblocks(g.volh), c->stream);
       } else {
         launch_mtil_pass1(sloppy, g, false, B.t, B.p, gauge_of(c, sloppy), ainv_of(c, sloppy), op, c->dcg,
-                          c->stream, nb, dkap);
+                          c->stream, nb, dkap, AlphaFin{}, true);
         launch_mtil_pass2(sloppy, g, false, B.q, B.t, B.p, gauge_of(c, sloppy), aee_of(c, sloppy), op, c->red,
-                          nullptr, c->dcg, c->stream, nb, drho, dkap, true);
+                          nullptr, c->dcg, c->stream, nb, drho, dkap, true, true);
         launch_mtil_pass1(sloppy, g, true, B.t, B.q, gauge_of(c, sloppy), ainv_of(c, sloppy), op, c->dcg,
-                          c->stream, nb, dkap, AlphaFin{c->red.partial, c->red.maxblocks, c->dcg});
-        launch_cg_pass4(sloppy, g, B.t, B.q, gauge_of(c, sloppy), aee_of(c, sloppy), op, B.p, B.xs, B.rs, c->red,
-                        c->dcg, c->stream, nb, true, drho, dkap, true);
+                          c->stream, nb, dkap, AlphaFin{c->red.partial, c->red.maxblocks, c->dcg}, true);
+        launch_cg_pass4(sloppy, g, B.t, B.q, gauge_of(c, sloppy), aee_of(c, sloppy), op, B.rs, c->red, c->dcg,
+                        c->stream, nb, drho, dkap, true, true);
         launch_cg_step(c->red, c->dcg, nb, nblocks(g.volh), c->stream);
       }
-      launch_cg_pupdate(sloppy, g, B.p, B.rs, c->dcg, c->stream, nb);
+      launch_cg_pupdate(sloppy, g, B.p, B.rs, c->dcg, c->stream, nb, B.xs, expect, true);
     }
     launches += 6 * batch;
     CKL();

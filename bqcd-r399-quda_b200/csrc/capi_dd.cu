@@ -752,7 +752,7 @@ int bqcdg_dd_solve(bqcdg_dd* dd, double* x, const double* b, const bqcdg_params*
       if (st || (st = dd_reduce(dd, nsb, dcg, 2))) return st;
       // x += alpha p of this iteration if it ran, p = r + beta p if the solve goes on
       for (int s = 0; s < n; s++)
-        launch_cg_pupdate(P, dd->slabs[s]->g, sp[s], rs[s], dcg, dd->stream, 1, xs[s], iter0 + k + 1);
+        launch_cg_pupdate(P, dd->slabs[s]->g, sp[s], rs[s], dcg, dd->stream, 1, xs[s], CgExpect{{iter0 + k + 1}});
       CKL();
       launches += 4 * (n + nparts * n) + 2 * (dd->nccl ? 2 : 1) + n;
     }

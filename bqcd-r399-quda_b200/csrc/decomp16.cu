@@ -254,8 +254,7 @@ __global__ void __launch_bounds__(kBlock) k_dd16_pack(Geom g, int V3h, int sf, i
 __device__ __forceinline__ void dd_apply_total(CgScalars* cg, double tot, double* out, int mode) {
   if (mode == 0) *out = tot;
   else if (mode == 1) {
-    cg->paap = tot;
-    cg->alpha = cg->rtr / tot;
+    cg_set_alpha(cg, tot);
   } else {
     cg_scalar_step(cg, tot);
   }

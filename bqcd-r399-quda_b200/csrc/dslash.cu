@@ -167,29 +167,40 @@ __global__ void __launch_bounds__(kBlock, Occ<P>::min_blocks) k_pass1(Geom g, Sp
                                                   CloverPtr ainv, int has_clover, double hval, const CgScalars* cg,
                                                   int nr, double kappa, const double* kappa_rhs, AlphaFin fin) {
   using R = typename SpinorView<P>::R;
-  const Tile tl = tile(nr);
-  if (cg && cg[tl.rhs].done) return;  // retired right-hand side
-  if (fin.partial && tl.sb == 0) {
-    // alpha of the k_pass2 before (launched with defer_alpha); the first
-    // CTAs of a launch run this while the others start on their sites
+  const Tile tl = tile(nr, fin.partial ? 1 : 0);
+  if (cg && cg[tl.rhs].done) {  // retired right-hand side
+    chain_wait();
+    return;
+  }
+  if (tl.sb < 0) {
+    // alpha of the k_pass2 before (launched with defer_alpha): one CTA more
+    // per right-hand side, first in the launch
+    chain_wait();
     double tot[1];
-    final_sum<1>(fin.partial + (size_t)tl.rhs * kRedVals * fin.stride, fin.stride, tl.nsb, tot);
+    final_sum<1>(after_wait(fin.partial) + (size_t)tl.rhs * kRedVals * fin.stride, fin.stride, tl.nsb, tot);
     if (threadIdx.x == 0) {
-      CgScalars* c = fin.cg + tl.rhs;
-      c->paap = tot[0];
-      c->alpha = c->rtr / tot[0];
+      cg_set_alpha(fin.cg + tl.rhs, tot[0]);
     }
+    return;
   }
   const int i = tl.i;
-  if (i >= g.volh) return;
+  if (i >= g.volh) {
+    chain_wait();
+    return;
+  }
   auto in = sview<P>(rhs_of(inp, tl.rhs), g.stride);
   auto out = sview<P>(rhs_of(outp, tl.rhs), g.stride);
   auto U = gview<P>(gauge, g);
   Site st = site_coords(g, i, 1);
   Spinor<R> b;
   zero(b);
-  if constexpr (P == Prec::F16) wilson_hop_lf<DAG>(g, 1, i, st, in, U, b);
-  else wilson_hop<P, DAG>(g, 1, i, st, in, U, b);
+  if constexpr (P == Prec::F16) {
+    wilson_hop_lf<DAG>(g, 1, i, st, in, U, b);  // waits (chain_wait) once its links are requested
+  } else {
+    chain_wait();
+    in = after_wait(in);
+    wilson_hop<P, DAG>(g, 1, i, st, in, U, b);
+  }
   R osc = 1;  // a common factor of the output, folded into its storage scale
   if (has_clover) {
     Spinor<R> y;
@@ -203,12 +214,13 @@ __global__ void __launch_bounds__(kBlock, Occ<P>::min_blocks) k_pass1(Geom g, Sp
 
 void launch_mtil_pass1(Prec p, const Geom& g, bool dag, SpinorPtr out_o, SpinorPtr in_e, const void* gauge,
                        CloverPtr ainv_oo, const OpParams& op, const CgScalars* cg, cudaStream_t s, int nr,
-                       const double* kappa_rhs, AlphaFin fin) {
-  dim3 grid(nblocks(g.volh) * nr);
+                       const double* kappa_rhs, AlphaFin fin, bool chain) {
+  dim3 grid((nblocks(g.volh) + (fin.partial ? 1 : 0)) * nr);
   int hc = op.csw_kappa != 0.0;
   double hv = dag ? op.h : -op.h;
 #define P1(PP, D, K) \
-  k_pass1<PP, D, K><<<grid, kBlock, 0, s>>>(g, out_o, in_e, gauge, ainv_oo, hc, hv, cg, nr, op.kappa, kappa_rhs, fin)
+  launch_chain(chain, k_pass1<PP, D, K>, grid, kBlock, s, g, out_o, in_e, gauge, ainv_oo, hc, hv, cg, nr, op.kappa, \
+               kappa_rhs, fin)
 #define P1K(PP, D) if (g.clover_t) P1(PP, D, true); else P1(PP, D, false);
   if (p == Prec::F64) { if (dag) { P1K(Prec::F64, true) } else { P1K(Prec::F64, false) } }
   else if (p == Prec::F32) { if (dag) { P1K(Prec::F32, true) } else { P1K(Prec::F32, false) } }
@@ -221,8 +233,10 @@ void launch_mtil_pass1(Prec p, const Geom& g, bool dag, SpinorPtr out_o, SpinorP
 // (+ i h' g5 x for Wilson, h_mult.F90:27-49), + rho x  (m_tilde.F90:63-73,
 // w_mult.F90:39).  The site-local terms come first and the hop sum is added
 // onto them, so the clover block and x are dead before the neighbour gathers
-// start; b is applied inside the hop sum and the storage scales of x and A_ee
-// as one factor, so no field is rescaled component by component.
+// start (x was written before the launch that writes t, so in a chained launch
+// they come before chain_wait); b is applied inside the hop sum and the storage
+// scales of x and A_ee as one factor, so no field is rescaled component by
+// component.
 template <Prec P, bool DAG, bool KT>
 __device__ __forceinline__ void pass2_core(const Geom& g, int i, const SpinorView<P>& t, const SpinorView<P>& xin,
                                            const GaugeView<P>& U, const CloverPtr& aee, int has_clover, double bcoef,
@@ -260,8 +274,12 @@ __device__ __forceinline__ void pass2_core(const Geom& g, int i, const SpinorVie
     }
   }
   const Site st = site_coords(g, i, 0);
-  if constexpr (P == Prec::F16) wilson_hop_lf<DAG>(g, 0, i, st, t, U, out, (R)bcoef);
-  else wilson_hop<P, DAG>(g, 0, i, st, t, U, out, (R)bcoef);
+  if constexpr (P == Prec::F16) {
+    wilson_hop_lf<DAG>(g, 0, i, st, t, U, out, (R)bcoef);  // waits (chain_wait) once its links are requested
+  } else {
+    chain_wait();
+    wilson_hop<P, DAG>(g, 0, i, st, after_wait(t), U, out, (R)bcoef);
+  }
 }
 
 template <Prec P, bool DAG, bool REDUCE, bool KT>
@@ -272,7 +290,10 @@ __global__ void __launch_bounds__(kBlock, Occ<P>::min_blocks2) k_pass2(Geom g, S
                                                   const double* kappa_rhs, bool defer_alpha) {
   using R = typename SpinorView<P>::R;
   const Tile tl = tile(nr);
-  if (cg && cg[tl.rhs].done) return;  // retired right-hand side
+  if (cg && cg[tl.rhs].done) {  // retired right-hand side
+    chain_wait();
+    return;
+  }
   if (rho_rhs) rho = rho_rhs[tl.rhs];   // a shift per right-hand side
   if (kappa_rhs) {                       // a hopping parameter per right-hand side
     kappa = kappa_rhs[tl.rhs];
@@ -294,6 +315,8 @@ __global__ void __launch_bounds__(kBlock, Occ<P>::min_blocks2) k_pass2(Geom g, S
 #pragma unroll
         for (int c = 0; c < 3; c++) acc[0] += (double)norm2(o.c[s][c]);
     }
+  } else {
+    chain_wait();
   }
   if (REDUCE) {
     double* part = red.partial + (size_t)tl.rhs * kRedVals * red.maxblocks;
@@ -307,9 +330,7 @@ __global__ void __launch_bounds__(kBlock, Occ<P>::min_blocks2) k_pass2(Geom g, S
       if (threadIdx.x == 0) {
         if (norm_out) norm_out[tl.rhs] = tot[0];
         if (cg) {
-          CgScalars* c = cg + tl.rhs;
-          c->paap = tot[0];
-          c->alpha = c->rtr / tot[0];
+          cg_set_alpha(cg + tl.rhs, tot[0]);
         }
         red.counter[tl.rhs] = 0;
       }
@@ -320,7 +341,7 @@ __global__ void __launch_bounds__(kBlock, Occ<P>::min_blocks2) k_pass2(Geom g, S
 void launch_mtil_pass2(Prec p, const Geom& g, bool dag, SpinorPtr out_e, SpinorPtr t_o, SpinorPtr in_e,
                        const void* gauge, CloverPtr a_ee, const OpParams& op, RedScratch red, double* norm_out,
                        CgScalars* cg, cudaStream_t s, int nr, const double* rho_rhs, const double* kappa_rhs,
-                       bool defer_alpha) {
+                       bool defer_alpha, bool chain) {
   dim3 grid(nblocks(g.volh) * nr);
   int hc = op.csw_kappa != 0.0;
   double bcoef = -op.kappa * op.kappa / (1.0 + op.h * op.h);
@@ -328,8 +349,8 @@ void launch_mtil_pass2(Prec p, const Geom& g, bool dag, SpinorPtr out_e, SpinorP
   bool reduce = norm_out != nullptr || cg != nullptr;
   defer_alpha = defer_alpha && cg && !norm_out;  // only alpha can wait for the next pass
 #define P2(PP, D, RR, K)                                                                                        \
-  k_pass2<PP, D, RR, K><<<grid, kBlock, 0, s>>>(g, out_e, t_o, in_e, gauge, a_ee, hc, bcoef, hv, op.rho, red, \
-                                                norm_out, cg, nr, rho_rhs, op.kappa, kappa_rhs, defer_alpha)
+  launch_chain(chain, k_pass2<PP, D, RR, K>, grid, kBlock, s, g, out_e, t_o, in_e, gauge, a_ee, hc, bcoef, hv,  \
+               op.rho, red, norm_out, cg, nr, rho_rhs, op.kappa, kappa_rhs, defer_alpha)
 #define P2R(PP, D)                                         \
   if (g.clover_t) {                                        \
     if (reduce) P2(PP, D, true, true); else P2(PP, D, false, true);   \
@@ -357,17 +378,20 @@ struct XR<Prec::F32> {
   using View = SpinorView<Prec::F32>;
 };
 
-template <Prec P, Prec XP, bool XUPD, bool KT>
+template <Prec P, Prec XP, bool KT>
 __global__ void __launch_bounds__(kBlock, Occ<P>::min_blocks2) k_cg_pass4(Geom g, SpinorPtr tp, SpinorPtr qp, const void* gauge,
                                                      CloverPtr aee, int has_clover, double bcoef, double hval,
-                                                     double rho, SpinorPtr pp, SpinorPtr xp, SpinorPtr rp,
+                                                     double rho, SpinorPtr rp,
                                                      RedScratch red, CgScalars* cgs, int nr, const double* rho_rhs,
                                                      double kappa, const double* kappa_rhs, bool defer_step) {
   using R = typename SpinorView<P>::R;
   using RX = typename SpinorView<XP>::R;
   const Tile tl = tile(nr);
   CgScalars* cg = cgs + tl.rhs;
-  if (cg->done) return;  // retired right-hand side
+  if (cg->done) {  // retired right-hand side
+    chain_wait();
+    return;
+  }
   if (rho_rhs) rho = rho_rhs[tl.rhs];  // a shift per right-hand side
   if (kappa_rhs) {                      // a hopping parameter per right-hand side
     kappa = kappa_rhs[tl.rhs];
@@ -379,28 +403,10 @@ __global__ void __launch_bounds__(kBlock, Occ<P>::min_blocks2) k_cg_pass4(Geom g
     auto t = sview<P>(rhs_of(tp, tl.rhs), g.stride);
     auto q = sview<P>(rhs_of(qp, tl.rhs), g.stride);
     auto U = gview<P>(gauge, g);
-    auto pv = sview<P>(rhs_of(pp, tl.rhs), g.stride);
-    auto xv = sview<XP>(rhs_of(xp, tl.rhs), g.stride);
     auto rv = sview<XP>(rhs_of(rp, tl.rhs), g.stride);
-    const RX a = (RX)cg->alpha;
-    if (XUPD) {
-      // x += alpha p first: alpha is known before the stencil, and x and p are
-      // then dead while the stencil runs (otherwise k_cg_pupdate does it)
-      Spinor<R> pl;
-      R psc;
-      pv.load_raw(i, pl, psc);
-      Spinor<RX> xl;
-      xv.load(i, xl);
-      const RX ap_sc = a * (RX)psc;  // alpha and the storage scale of p
-#pragma unroll
-      for (int s = 0; s < 4; s++)
-#pragma unroll
-        for (int c = 0; c < 3; c++)
-          xl.c[s][c] = xl.c[s][c] + ap_sc * mkc((RX)pl.c[s][c].x, (RX)pl.c[s][c].y);
-      xv.store(i, xl);
-    }
     Spinor<R> ap;
     pass2_core<P, true, KT>(g, i, t, q, U, aee, has_clover, bcoef, hval, rho, ap, kappa);
+    const RX a = (RX)cg->alpha;  // set by the launch before
     Spinor<RX> rl;
     rv.load(i, rl);
 #pragma unroll
@@ -411,6 +417,8 @@ __global__ void __launch_bounds__(kBlock, Occ<P>::min_blocks2) k_cg_pass4(Geom g
         acc[0] += (double)norm2(rl.c[s][c]);
       }
     rv.store(i, rl);
+  } else {
+    chain_wait();
   }
   double* part = red.partial + (size_t)tl.rhs * kRedVals * red.maxblocks;
   block_reduce_store<1>(acc, part, red.maxblocks, tl.sb);
@@ -429,72 +437,72 @@ __global__ void __launch_bounds__(kBlock, Occ<P>::min_blocks2) k_cg_pass4(Geom g
 constexpr int kStepBlock = 1024;
 __global__ void __launch_bounds__(kStepBlock) k_cg_step(RedScratch red, CgScalars* cgs, int nsb) {
   CgScalars* cg = cgs + blockIdx.x;
+  chain_wait();
   if (cg->done) return;  // k_cg_pass4 did not run for this right-hand side
   double tot[1];
-  final_sum<1>(red.partial + (size_t)blockIdx.x * kRedVals * red.maxblocks, red.maxblocks, nsb, tot);
+  final_sum<1>(after_wait(red.partial) + (size_t)blockIdx.x * kRedVals * red.maxblocks, red.maxblocks, nsb, tot);
   if (threadIdx.x == 0) cg_scalar_step(cg, tot[0]);
 }
 
 void launch_cg_step(RedScratch red, CgScalars* cg, int nr, int nsb, cudaStream_t s) {
-  k_cg_step<<<nr, kStepBlock, 0, s>>>(red, cg, nsb);
+  launch_chain(true, k_cg_step, dim3(nr), kStepBlock, s, red, cg, nsb);
 }
 
 void launch_cg_pass4(Prec p, const Geom& g, SpinorPtr t_o, SpinorPtr q_e, const void* gauge, CloverPtr a_ee,
-                     const OpParams& op, SpinorPtr pvec, SpinorPtr x, SpinorPtr r, RedScratch red, CgScalars* cg,
-                     cudaStream_t s, int nr, bool xupd, const double* rho_rhs, const double* kappa_rhs,
-                     bool defer_step) {
+                     const OpParams& op, SpinorPtr r, RedScratch red, CgScalars* cg, cudaStream_t s, int nr,
+                     const double* rho_rhs, const double* kappa_rhs, bool defer_step, bool chain) {
   dim3 grid(nblocks(g.volh) * nr);
   int hc = op.csw_kappa != 0.0;
   double bcoef = -op.kappa * op.kappa / (1.0 + op.h * op.h);
   double hv = -op.h;  // mtil_dag
-#define P4(PP, XX, XU, K)                                                                                   \
-  k_cg_pass4<PP, XX, XU, K><<<grid, kBlock, 0, s>>>(g, t_o, q_e, gauge, a_ee, hc, bcoef, hv, op.rho, pvec, x, r, \
-                                                    red, cg, nr, rho_rhs, op.kappa, kappa_rhs, defer_step)
-#define P4K(PP, XX, XU) if (g.clover_t) P4(PP, XX, XU, true); else P4(PP, XX, XU, false);
-  if (p == Prec::F64) { if (xupd) { P4K(Prec::F64, Prec::F64, true) } else { P4K(Prec::F64, Prec::F64, false) } }
-  else if (p == Prec::F32) { if (xupd) { P4K(Prec::F32, Prec::F32, true) } else { P4K(Prec::F32, Prec::F32, false) } }
-  else { if (xupd) { P4K(Prec::F16, Prec::F32, true) } else { P4K(Prec::F16, Prec::F32, false) } }
+#define P4(PP, XX, K)                                                                                         \
+  launch_chain(chain, k_cg_pass4<PP, XX, K>, grid, kBlock, s, g, t_o, q_e, gauge, a_ee, hc, bcoef, hv, op.rho, r, \
+               red, cg, nr, rho_rhs, op.kappa, kappa_rhs, defer_step)
+#define P4K(PP, XX) if (g.clover_t) P4(PP, XX, true); else P4(PP, XX, false);
+  if (p == Prec::F64) { P4K(Prec::F64, Prec::F64) }
+  else if (p == Prec::F32) { P4K(Prec::F32, Prec::F32) }
+  else { P4K(Prec::F16, Prec::F32) }
 #undef P4K
 #undef P4
 }
 
-// p = r + beta p   (sc_xpby, cg.F90:116), and, when x is given, the x += alpha p
-// of the same iteration (cg.F90:101), which then runs here instead of in the
-// stencil pass: this kernel reads p anyway.  The launch belongs to iteration
-// `expect`: x is updated iff that iteration ran (its k_cg_pass4 counted it),
-// p iff the solve goes on; so the update of the last iteration is not lost
-// when the solver stops, and no x update is applied twice.
-template <Prec P, Prec RP, bool XUPD>
+// p = r + beta p   (sc_xpby, cg.F90:116) and the x += alpha p of the same
+// iteration (cg.F90:101), which runs here instead of in the stencil pass: this
+// kernel reads p anyway.  The launch belongs to iteration `expect` of each
+// right-hand side: x is updated iff that iteration ran (its alpha was set),
+// p iff the solve goes on; so the update of the last iteration is not
+// lost when the solver stops, and no x update is applied twice.  Everything
+// but beta and the stop flag was written before the CG step, so p, x and r are
+// requested before chain_wait.
+template <Prec P, Prec RP>
 __global__ void __launch_bounds__(kBlock) k_cg_pupdate(Geom g, SpinorPtr pp, SpinorPtr rp, SpinorPtr xp,
-                                                       const CgScalars* cgs, int nr, int expect) {
+                                                       const CgScalars* cgs, int nr, CgExpect expect) {
   using R = typename SpinorView<P>::R;
   using RR = typename SpinorView<RP>::R;
   const Tile tl = tile(nr);
   const CgScalars* cg = cgs + tl.rhs;
-  const bool upd_p = !cg->done;
-  const bool upd_x = XUPD && cg->iter == expect;
-  if (!upd_p && !upd_x) return;
   const int i = tl.i;
-  if (i >= g.volh) return;
+  if (cg->live != expect.n[tl.rhs] || i >= g.volh) {  // retired before this iteration
+    chain_wait();
+    return;
+  }
   auto pv = sview<P>(rhs_of(pp, tl.rhs), g.stride);
+  auto xv = sview<RP>(rhs_of(xp, tl.rhs), g.stride);
+  auto rv = sview<RP>(rhs_of(rp, tl.rhs), g.stride);
   Spinor<R> pl;
   R psc;
+  Spinor<RR> xl, rl;
   pv.load_raw(i, pl, psc);
-  if (XUPD && upd_x) {
-    auto xv = sview<RP>(rhs_of(xp, tl.rhs), g.stride);
-    Spinor<RR> xl;
-    xv.load(i, xl);
-    const RR a = (RR)cg->alpha * (RR)psc;
-#pragma unroll
-    for (int s = 0; s < 4; s++)
-#pragma unroll
-      for (int c = 0; c < 3; c++) xl.c[s][c] = xl.c[s][c] + a * mkc((RR)pl.c[s][c].x, (RR)pl.c[s][c].y);
-    xv.store(i, xl);
-  }
-  if (!upd_p) return;
-  auto rv = sview<RP>(rhs_of(rp, tl.rhs), g.stride);
-  Spinor<RR> rl;
+  xv.load(i, xl);
   rv.load(i, rl);
+  const RR a = (RR)cg->alpha * (RR)psc;
+  chain_wait();
+#pragma unroll
+  for (int s = 0; s < 4; s++)
+#pragma unroll
+    for (int c = 0; c < 3; c++) xl.c[s][c] = xl.c[s][c] + a * mkc((RR)pl.c[s][c].x, (RR)pl.c[s][c].y);
+  xv.store(i, xl);
+  if (cg->done) return;
   const R b = (R)cg->beta * psc;
 #pragma unroll
   for (int s = 0; s < 4; s++)
@@ -504,13 +512,12 @@ __global__ void __launch_bounds__(kBlock) k_cg_pupdate(Geom g, SpinorPtr pp, Spi
 }
 
 void launch_cg_pupdate(Prec p, const Geom& g, SpinorPtr pvec, SpinorPtr r, CgScalars* cg, cudaStream_t s, int nr,
-                       SpinorPtr x, int expect) {
+                       SpinorPtr x, const CgExpect& expect, bool chain) {
   dim3 grid(nblocks(g.volh) * nr);
-  const bool xu = x.v != nullptr;
-#define PU(PP, RR, XU) k_cg_pupdate<PP, RR, XU><<<grid, kBlock, 0, s>>>(g, pvec, r, x, cg, nr, expect)
-  if (p == Prec::F64) { if (xu) PU(Prec::F64, Prec::F64, true); else PU(Prec::F64, Prec::F64, false); }
-  else if (p == Prec::F32) { if (xu) PU(Prec::F32, Prec::F32, true); else PU(Prec::F32, Prec::F32, false); }
-  else { if (xu) PU(Prec::F16, Prec::F32, true); else PU(Prec::F16, Prec::F32, false); }
+#define PU(PP, RR) launch_chain(chain, k_cg_pupdate<PP, RR>, grid, kBlock, s, g, pvec, r, x, cg, nr, expect)
+  if (p == Prec::F64) PU(Prec::F64, Prec::F64);
+  else if (p == Prec::F32) PU(Prec::F32, Prec::F32);
+  else PU(Prec::F16, Prec::F32);
 #undef PU
 }
 

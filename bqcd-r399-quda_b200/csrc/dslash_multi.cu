@@ -27,11 +27,12 @@ struct GTile {
   int nsb;
   int i;
 };
-__device__ __forceinline__ GTile gtile(int ng) {
+// (the first `extra` site blocks of the launch are for other work: sb < 0)
+__device__ __forceinline__ GTile gtile(int ng, int extra = 0) {
   GTile t;
   t.grp = blockIdx.x % ng;
-  t.sb = blockIdx.x / ng;
-  t.nsb = gridDim.x / ng;
+  t.sb = (int)(blockIdx.x / ng) - extra;
+  t.nsb = gridDim.x / ng - extra;
   t.i = t.sb * blockDim.x + threadIdx.x;
   return t;
 }
@@ -195,26 +196,32 @@ __global__ void __launch_bounds__(kBlock, OccN<NB>::min_blocks)
     k_pass1_n(Geom g, SpinorPtr outp, SpinorPtr inp, const void* gauge, CloverPtr ainv, int has_clover, double hval,
               const CgScalars* cg, int nr, int ng, AlphaFin fin) {
   using R = typename SpinorView<P>::R;
-  const GTile tl = gtile(ng);
+  const GTile tl = gtile(ng, fin.partial ? 1 : 0);
   const int rhs0 = tl.grp * NB;
   bool act[NB];
-  if (!group_live<NB>(cg, rhs0, nr, act)) return;
-  if (fin.partial && tl.sb == 0) {
+  if (!group_live<NB>(cg, rhs0, nr, act)) {
+    chain_wait();
+    return;
+  }
+  if (tl.sb < 0) {
     // alpha of the k_pass2_n before (defer_alpha), as in k_pass1
+    chain_wait();
     double tot[NB];
-    final_sum<NB>(fin.partial + (size_t)rhs0 * kRedVals * fin.stride, kRedVals * fin.stride, tl.nsb, tot);
+    final_sum<NB>(after_wait(fin.partial) + (size_t)rhs0 * kRedVals * fin.stride, kRedVals * fin.stride, tl.nsb, tot);
     if (threadIdx.x == 0) {
 #pragma unroll
       for (int r = 0; r < NB; r++) {
         if (!act[r]) continue;
-        CgScalars* c = fin.cg + rhs0 + r;
-        c->paap = tot[r];
-        c->alpha = c->rtr / tot[r];
+        cg_set_alpha(fin.cg + rhs0 + r, tot[r]);
       }
     }
+    return;
   }
   const int i = tl.i;
-  if (i >= g.volh) return;
+  if (i >= g.volh) {
+    chain_wait();
+    return;
+  }
   SpinorView<P> in[NB];
 #pragma unroll
   for (int r = 0; r < NB; r++) in[r] = sview<P>(rhs_of(inp, rhs0 + r), g.stride);
@@ -223,6 +230,9 @@ __global__ void __launch_bounds__(kBlock, OccN<NB>::min_blocks)
   Spinor<R> b[NB];
 #pragma unroll
   for (int r = 0; r < NB; r++) zero(b[r]);
+  chain_wait();
+#pragma unroll
+  for (int r = 0; r < NB; r++) in[r] = after_wait(in[r]);
   wilson_hop_n<P, DAG, NB>(g, 1, i, st, in, act, U, b, (R)1);
   R osc = 1;  // a common factor of the outputs, folded into their storage scale
   if (has_clover) {
@@ -239,13 +249,13 @@ __global__ void __launch_bounds__(kBlock, OccN<NB>::min_blocks)
 
 void launch_mtil_pass1_n(Prec p, const Geom& g, bool dag, SpinorPtr out_o, SpinorPtr in_e, const void* gauge,
                          CloverPtr ainv_oo, const OpParams& op, const CgScalars* cg, cudaStream_t s, int nr,
-                         int nbt, AlphaFin fin) {
+                         int nbt, AlphaFin fin, bool chain) {
   const int ng = (nr + nbt - 1) / nbt;
-  dim3 grid(nblocks(g.volh) * ng);
+  dim3 grid((nblocks(g.volh) + (fin.partial ? 1 : 0)) * ng);
   int hc = op.csw_kappa != 0.0;
   double hv = dag ? op.h : -op.h;
 #define P1N(PP, D, N) \
-  k_pass1_n<PP, D, N><<<grid, kBlock, 0, s>>>(g, out_o, in_e, gauge, ainv_oo, hc, hv, cg, nr, ng, fin)
+  launch_chain(chain, k_pass1_n<PP, D, N>, grid, kBlock, s, g, out_o, in_e, gauge, ainv_oo, hc, hv, cg, nr, ng, fin)
 #define P1NB(PP, N) \
   if (dag) P1N(PP, true, N); else P1N(PP, false, N)
   if (p == Prec::F32) { if (nbt == 2) { P1NB(Prec::F32, 2); } else { P1NB(Prec::F32, 4); } }
@@ -301,7 +311,11 @@ __device__ __forceinline__ void pass2_core_n(const Geom& g, int i, const SpinorV
     }
   }
   const Site st = site_coords(g, i, 0);
-  wilson_hop_n<P, DAG, NB>(g, 0, i, st, t, act, U, out, (R)bcoef);
+  chain_wait();  // t is written by the launch before, x and the clover blocks earlier
+  SpinorView<P> tw[NB];
+#pragma unroll
+  for (int r = 0; r < NB; r++) tw[r] = after_wait(t[r]);
+  wilson_hop_n<P, DAG, NB>(g, 0, i, st, tw, act, U, out, (R)bcoef);
 }
 
 // the shifts of the group's right-hand sides
@@ -323,7 +337,10 @@ __global__ void __launch_bounds__(kBlock, OccN<NB>::min_blocks)
   const GTile tl = gtile(ng);
   const int rhs0 = tl.grp * NB;
   bool act[NB];
-  if (!group_live<NB>(cg, rhs0, nr, act)) return;
+  if (!group_live<NB>(cg, rhs0, nr, act)) {
+    chain_wait();
+    return;
+  }
   double rh[NB];
   group_rho<NB>(rho, rho_rhs, rhs0, act, rh);
   const int i = tl.i;
@@ -348,6 +365,8 @@ __global__ void __launch_bounds__(kBlock, OccN<NB>::min_blocks)
 #pragma unroll
         for (int c = 0; c < 3; c++) acc[r] += (double)norm2(o[r].c[s][c]);
     }
+  } else {
+    chain_wait();
   }
   // value r of the group goes to the partial slot of RHS rhs0 + r
   double* part = red.partial + (size_t)rhs0 * kRedVals * red.maxblocks;
@@ -359,9 +378,7 @@ __global__ void __launch_bounds__(kBlock, OccN<NB>::min_blocks)
 #pragma unroll
       for (int r = 0; r < NB; r++) {
         if (!act[r]) continue;
-        CgScalars* c = cg + rhs0 + r;
-        c->paap = tot[r];
-        c->alpha = c->rtr / tot[r];
+        cg_set_alpha(cg + rhs0 + r, tot[r]);
       }
       red.counter[rhs0] = 0;
     }
@@ -370,32 +387,34 @@ __global__ void __launch_bounds__(kBlock, OccN<NB>::min_blocks)
 
 void launch_mtil_pass2_n(Prec p, const Geom& g, SpinorPtr out_e, SpinorPtr t_o, SpinorPtr in_e, const void* gauge,
                          CloverPtr a_ee, const OpParams& op, RedScratch red, CgScalars* cg, cudaStream_t s, int nr,
-                         const double* rho_rhs, int nbt, bool defer_alpha) {
+                         const double* rho_rhs, int nbt, bool defer_alpha, bool chain) {
   const int ng = (nr + nbt - 1) / nbt;
   dim3 grid(nblocks(g.volh) * ng);
   int hc = op.csw_kappa != 0.0;
   double bcoef = -op.kappa * op.kappa;  // h = 0
 #define P2N(PP, N)                                                                                          \
-  k_pass2_n<PP, N><<<grid, kBlock, 0, s>>>(g, out_e, t_o, in_e, gauge, a_ee, hc, bcoef, op.rho, red, cg, nr, ng, \
-                                           rho_rhs, defer_alpha)
+  launch_chain(chain, k_pass2_n<PP, N>, grid, kBlock, s, g, out_e, t_o, in_e, gauge, a_ee, hc, bcoef, op.rho, red, \
+               cg, nr, ng, rho_rhs, defer_alpha)
   if (p == Prec::F32) { if (nbt == 2) P2N(Prec::F32, 2); else P2N(Prec::F32, 4); }
   else { if (nbt == 2) P2N(Prec::F16, 2); else P2N(Prec::F16, 4); }
 #undef P2N
 }
 
 // CG-fused second half of mtil_dag for NB right-hand sides (k_cg_pass4 of
-// dslash.cu, x updated here): x_r += alpha_r p_r, Ap_r = A_ee q_r + b D_eo t_r
-// + rho_r q_r, r_r -= alpha_r Ap_r, and the CG scalars from |r_r|^2
+// dslash.cu): Ap_r = A_ee q_r + b D_eo t_r + rho_r q_r, r_r -= alpha_r Ap_r, and the CG scalars from |r_r|^2
 template <Prec P, int NB>
 __global__ void __launch_bounds__(kBlock, OccN<NB>::min_blocks)
     k_cg_pass4_n(Geom g, SpinorPtr tp, SpinorPtr qp, const void* gauge, CloverPtr aee, int has_clover, double bcoef,
-                 double rho, SpinorPtr pp, SpinorPtr xp, SpinorPtr rp, RedScratch red, CgScalars* cgs, int nr, int ng,
+                 double rho, SpinorPtr rp, RedScratch red, CgScalars* cgs, int nr, int ng,
                  const double* rho_rhs, bool defer_step) {
   using R = typename SpinorView<P>::R;
   const GTile tl = gtile(ng);
   const int rhs0 = tl.grp * NB;
   bool act[NB];
-  if (!group_live<NB>(cgs, rhs0, nr, act)) return;
+  if (!group_live<NB>(cgs, rhs0, nr, act)) {
+    chain_wait();
+    return;
+  }
   double rh[NB];
   group_rho<NB>(rho, rho_rhs, rhs0, act, rh);
   const int i = tl.i;
@@ -403,25 +422,6 @@ __global__ void __launch_bounds__(kBlock, OccN<NB>::min_blocks)
 #pragma unroll
   for (int r = 0; r < NB; r++) acc[r] = 0.0;
   if (i < g.volh) {
-    // x += alpha p first: alpha is known before the stencil, and x and p are
-    // then dead while the stencil runs
-#pragma unroll
-    for (int r = 0; r < NB; r++) {
-      if (!act[r]) continue;
-      const auto pv = sview<P>(rhs_of(pp, rhs0 + r), g.stride);
-      const auto xv = sview<Prec::F32>(rhs_of(xp, rhs0 + r), g.stride);
-      Spinor<R> pl;
-      R psc;
-      pv.load_raw(i, pl, psc);
-      Spinor<float> xl;
-      xv.load(i, xl);
-      const float ap_sc = (float)cgs[rhs0 + r].alpha * (float)psc;
-#pragma unroll
-      for (int s = 0; s < 4; s++)
-#pragma unroll
-        for (int c = 0; c < 3; c++) xl.c[s][c] = xl.c[s][c] + ap_sc * mkc((float)pl.c[s][c].x, (float)pl.c[s][c].y);
-      xv.store(i, xl);
-    }
     SpinorView<P> t[NB], q[NB];
 #pragma unroll
     for (int r = 0; r < NB; r++) {
@@ -446,6 +446,8 @@ __global__ void __launch_bounds__(kBlock, OccN<NB>::min_blocks)
         }
       rv.store(i, rl);
     }
+  } else {
+    chain_wait();
   }
   double* part = red.partial + (size_t)rhs0 * kRedVals * red.maxblocks;
   block_reduce_store<NB>(acc, part, kRedVals * red.maxblocks, tl.sb);
@@ -464,15 +466,15 @@ __global__ void __launch_bounds__(kBlock, OccN<NB>::min_blocks)
 }
 
 void launch_cg_pass4_n(Prec p, const Geom& g, SpinorPtr t_o, SpinorPtr q_e, const void* gauge, CloverPtr a_ee,
-                       const OpParams& op, SpinorPtr pvec, SpinorPtr x, SpinorPtr r, RedScratch red, CgScalars* cg,
-                       cudaStream_t s, int nr, const double* rho_rhs, int nbt, bool defer_step) {
+                       const OpParams& op, SpinorPtr r, RedScratch red, CgScalars* cg, cudaStream_t s, int nr,
+                       const double* rho_rhs, int nbt, bool defer_step, bool chain) {
   const int ng = (nr + nbt - 1) / nbt;
   dim3 grid(nblocks(g.volh) * ng);
   int hc = op.csw_kappa != 0.0;
   double bcoef = -op.kappa * op.kappa;  // h = 0
 #define P4N(PP, N)                                                                                              \
-  k_cg_pass4_n<PP, N><<<grid, kBlock, 0, s>>>(g, t_o, q_e, gauge, a_ee, hc, bcoef, op.rho, pvec, x, r, red, cg, nr, \
-                                              ng, rho_rhs, defer_step)
+  launch_chain(chain, k_cg_pass4_n<PP, N>, grid, kBlock, s, g, t_o, q_e, gauge, a_ee, hc, bcoef, op.rho, r, red, cg, \
+               nr, ng, rho_rhs, defer_step)
   if (p == Prec::F32) { if (nbt == 2) P4N(Prec::F32, 2); else P4N(Prec::F32, 4); }
   else { if (nbt == 2) P4N(Prec::F16, 2); else P4N(Prec::F16, 4); }
 #undef P4N

@@ -35,23 +35,25 @@ struct RedScratch {
   int maxblocks = 0;
 };
 
-// scalars of a CG kept in device memory (no host round trip per iteration)
-struct CgScalars {
+// scalars of a CG kept in device memory (no host round trip per iteration).
+// alpha and live, which the second half of an iteration reads, have a cache
+// line of their own: the CG step writes the first line while k_cg_pupdate,
+// launched behind it (launch_chain), already reads the second.
+struct alignas(256) CgScalars {
   double rtr;       // |r|^2 after the latest update
   double rtr_old;   // |r|^2 of the previous iteration
-  double paap;      // p.(A p) = |M p|^2
-  double alpha;
   double beta;
   double stop_rtr;  // converged when rtr <= stop_rtr
-  double ru_rtr;    // unused (kept for layout); see delta2/maxr2
+  double delta2;    // sloppy solver: reliable update when rtr < delta2 * maxr2 (0: never)
+  double maxr2;     // largest |r|^2 since the last reliable update
   int iter;         // iterations completed
   int maxiter;
   int done;         // 0 running, 1 converged, 2 reliable update requested, 3 maxiter, 4 NaN
-  int pad;
-  double delta2;    // sloppy solver: reliable update when rtr < delta2 * maxr2 (0: never)
-  double maxr2;     // largest |r|^2 since the last reliable update
   int last_ru;      // iteration of the last reliable update
   int ru_every;     // also update after this many iterations without one (0: never)
+  alignas(128) double paap;  // p.(A p) = |M p|^2
+  double alpha;
+  int live;         // the iteration that alpha belongs to (iter + 1 when it was set)
 };
 
 struct OpParams {
@@ -59,6 +61,35 @@ struct OpParams {
   double csw_kappa;
   double h;
   double rho;
+};
+
+// A launch that may start while the kernel before it in the stream drains
+// (programmatic stream serialization), when chain is set.  Only for kernels
+// whose threads all call chain_wait (bqcdg_internal.cuh, which has the rules),
+// and only where the launch before does not write the links, the clover
+// fields or whatever else the kernel reads before chain_wait.  Without it
+// about 2.2 us pass between two launches; with it the next kernel's index
+// arithmetic, links, clover blocks and local spinor are on their way by then.
+// Mixed solves: 18.7 -> 12.9 ms at 16^3x32, 6.6 -> 4.6 ms at 10x6x14x18; FP64
+// CG: 9.0 -> 6.7 ms at 8^4, 173.4 -> 169.9 ms at 24^3x48; at 32^3x64, where a
+// launch takes 100 us, no change.
+template <typename... KP, typename... A>
+inline void launch_chain(bool chain, void (*k)(KP...), dim3 grid, int block, cudaStream_t s, A... a) {
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(block);
+  cfg.stream = s;
+  cfg.attrs = &at;
+  cfg.numAttrs = chain ? 1 : 0;
+  cudaLaunchKernelEx(&cfg, k, KP(a)...);  // an error is seen by the caller's cudaGetLastError
+}
+
+// the iteration a k_cg_pupdate launch belongs to, per right-hand side
+struct CgExpect {
+  int n[kMaxRhs];
 };
 
 constexpr int kBlock = 128;
@@ -80,8 +111,7 @@ void launch_clover_mult_b(const Geom& g, double2* x, const double2* b, cudaStrea
 //  kappa_rhs also sets each right-hand side's hopping coefficient)
 // The |M~ p|^2 block partials that a k_pass2 launched with defer_alpha left
 // in red.partial (slot 0 of each RHS).  The k_pass1 launch after it, given
-// this, sums them in its first site block of each RHS, before its own sites,
-// and sets that RHS's paap and alpha = rtr / paap: the same fixed-order sum
+// this, sums them in one more CTA per RHS and sets that RHS's paap and alpha = rtr / paap: the same fixed-order sum
 // (final_sum) that k_pass2's last block would run, so alpha is bit for bit
 // the same, but no k_pass2 block waits for an arrival counter.
 struct AlphaFin {
@@ -91,20 +121,20 @@ struct AlphaFin {
 };
 void launch_mtil_pass1(Prec p, const Geom& g, bool dag, SpinorPtr out_o, SpinorPtr in_e, const void* gauge,
                        CloverPtr ainv_oo, const OpParams& op, const CgScalars* cg, cudaStream_t s, int nr = 1,
-                       const double* kappa_rhs = nullptr, AlphaFin fin = AlphaFin{});
+                       const double* kappa_rhs = nullptr, AlphaFin fin = AlphaFin{}, bool chain = false);
 // second half: out_e = A_ee in_e + b D_eo t_o (+ h term for Wilson) + rho in_e;
 // optional |out|^2 reduction into *norm_out (device), and CG alpha update
 void launch_mtil_pass2(Prec p, const Geom& g, bool dag, SpinorPtr out_e, SpinorPtr t_o, SpinorPtr in_e,
                        const void* gauge, CloverPtr a_ee, const OpParams& op, RedScratch red, double* norm_out,
                        CgScalars* cg, cudaStream_t s, int nr = 1, const double* rho_rhs = nullptr,
-                       const double* kappa_rhs = nullptr, bool defer_alpha = false);
+                       const double* kappa_rhs = nullptr, bool defer_alpha = false, bool chain = false);
 // CG-fused second half of mtil_dag: Ap = A_ee q + b D_eo t_o + rho q computed in
-// registers; x += alpha p, r -= alpha Ap, rtr = |r|^2.  Precision P for the
-// stencil fields, x/r in XP (F64 for the FP64 solver, F32 for the sloppy one)
+// registers; r -= alpha Ap, rtr = |r|^2 (x += alpha p follows in
+// k_cg_pupdate).  Precision P for the stencil fields, r in XP (F64 for the FP64 solver, F32 for the sloppy one)
 void launch_cg_pass4(Prec p, const Geom& g, SpinorPtr t_o, SpinorPtr q_e, const void* gauge, CloverPtr a_ee,
-                     const OpParams& op, SpinorPtr pvec, SpinorPtr x, SpinorPtr r, RedScratch red, CgScalars* cg,
-                     cudaStream_t s, int nr = 1, bool xupd = true, const double* rho_rhs = nullptr,
-                     const double* kappa_rhs = nullptr, bool defer_step = false);
+                     const OpParams& op, SpinorPtr r, RedScratch red, CgScalars* cg, cudaStream_t s, int nr = 1,
+                     const double* rho_rhs = nullptr, const double* kappa_rhs = nullptr, bool defer_step = false,
+                     bool chain = false);
 // With defer_step, k_cg_pass4 leaves its |r|^2 block partials in red.partial
 // and launch_cg_step, queued after it, sums them (one CTA per right-hand
 // side, the fixed-order final_sum) and takes the CG scalar step
@@ -117,21 +147,21 @@ void launch_cg_step(RedScratch red, CgScalars* cg, int nr, int nsb, cudaStream_t
 // register-blocked batched passes (dslash_multi.cu): one thread serves one
 // site of nbt (2 or 4) right-hand sides, so each link and clover block is
 // loaded and decoded once for all of them.  Sloppy precisions (F32, F16)
-// and h = 0 only; pass 2 is the non-dagger one with the CG alpha update, and
-// pass 4 updates x (cg required for both).
+// and h = 0 only; pass 2 is the non-dagger one with the CG alpha update (cg
+// required there and in pass 4).
 void launch_mtil_pass1_n(Prec p, const Geom& g, bool dag, SpinorPtr out_o, SpinorPtr in_e, const void* gauge,
                          CloverPtr ainv_oo, const OpParams& op, const CgScalars* cg, cudaStream_t s, int nr,
-                         int nbt, AlphaFin fin = AlphaFin{});
+                         int nbt, AlphaFin fin = AlphaFin{}, bool chain = false);
 void launch_mtil_pass2_n(Prec p, const Geom& g, SpinorPtr out_e, SpinorPtr t_o, SpinorPtr in_e, const void* gauge,
                          CloverPtr a_ee, const OpParams& op, RedScratch red, CgScalars* cg, cudaStream_t s, int nr,
-                         const double* rho_rhs, int nbt, bool defer_alpha = false);
+                         const double* rho_rhs, int nbt, bool defer_alpha = false, bool chain = false);
 void launch_cg_pass4_n(Prec p, const Geom& g, SpinorPtr t_o, SpinorPtr q_e, const void* gauge, CloverPtr a_ee,
-                       const OpParams& op, SpinorPtr pvec, SpinorPtr x, SpinorPtr r, RedScratch red, CgScalars* cg,
-                       cudaStream_t s, int nr, const double* rho_rhs, int nbt, bool defer_step = false);
-// p = r + beta p; with x given (xupd = false above, single RHS), also the
-// x += alpha p of iteration `expect` if that iteration ran
+                       const OpParams& op, SpinorPtr r, RedScratch red, CgScalars* cg, cudaStream_t s, int nr,
+                       const double* rho_rhs, int nbt, bool defer_step = false, bool chain = false);
+// p = r + beta p, and the x += alpha p of iteration expect.n[rhs] if that
+// iteration ran
 void launch_cg_pupdate(Prec p, const Geom& g, SpinorPtr pvec, SpinorPtr r, CgScalars* cg, cudaStream_t s,
-                       int nr = 1, SpinorPtr x = SpinorPtr{}, int expect = -1);
+                       int nr, SpinorPtr x, const CgExpect& expect, bool chain = false);
 
 // ---- block solver (blockcg.cu) ----
 // out[i * s + j] = <a_i, b_j> (FP64) for two blocks of s <= 16 FP32 fields

@@ -51,6 +51,13 @@ __device__ __forceinline__ CloverView<Prec::F16> cview<Prec::F16>(CloverPtr p, i
   return CloverView<Prec::F16>{(int4*)p.v, p.norm, stride};
 }
 
+// |M p|^2 is known: alpha of the iteration under way
+__device__ __forceinline__ void cg_set_alpha(CgScalars* cg, double paap) {
+  cg->paap = paap;
+  cg->alpha = cg->rtr / paap;
+  cg->live = cg->iter + 1;
+}
+
 // the scalar part of one CG iteration once |r|^2 of the new residual is
 // known (cg.F90:107-116), with the stop and reliable-update decisions of the
 // mixed-precision solver; run by one thread: of k_cg_step in the CG loop, of
