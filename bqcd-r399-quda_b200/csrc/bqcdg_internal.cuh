@@ -1026,65 +1026,58 @@ __device__ __forceinline__ void mul_ud(const Link<R>& u, const cx<R> h[2][3], cx
     }
 }
 
-// b += hscale * (sum over the 8 hops of the even/odd hopping term): out(parity
-// e, site i) from the field ``in`` of the opposite parity (d/D21.F90:29-77).
-// b is accumulated into, so a caller either zeroes it or starts it with the
-// site-local terms of its operator.
-// Every storage scale (int16 spinors and links), the boundary sign and hscale
-// are applied as one factor per hop, to the transported half spinor.
+// b += hscale * (the two hops of direction mu of the even/odd hopping term):
+// out(parity e, site i) from the field ``in`` of the opposite parity
+// (d/D21.F90:29-77).  Every storage scale (int16 spinors and links), the
+// boundary sign and hscale are applied as one factor per hop, to the
+// transported half spinor.  mu is a constant once inlined.
+template <Prec PS, bool DAG, typename UV>
+__device__ __forceinline__ void wilson_hop_mu(const Geom& g, int e, int i, const Site& st,
+                                              const SpinorView<PS>& in, const UV& U,
+                                              Spinor<typename SpinorView<PS>::R>& b,
+                                              typename SpinorView<PS>::R hscale, const int mu) {
+  using R = typename SpinorView<PS>::R;
+  const int o = 1 - e;
+#pragma unroll
+  for (int fb = 0; fb < 2; fb++) {
+    const bool fwd = fb == 0;
+    const int j = neighbour(g, st, i, mu, fwd);
+    cx<R> h[2][3], f[2][3];
+    R sc, lsc;
+    if (mu == 3) {
+      // (1 -+ gamma_4) keeps two spins: (3,4) for d, (1,2) for d_dag
+      in.load_pair_raw(j, fwd ? (DAG ? 0 : 2) : (DAG ? 2 : 0), h, sc);
+    } else if constexpr (PS == Prec::F16) {
+      float2 F[4][3];
+      in.load_biased(j, F, sc);
+      project_biased<DAG>(F, mu, fwd, h);
+    } else {
+      Spinor<R> p;
+      in.load_raw(j, p, sc);
+      project<R, DAG>(p, mu, fwd, h);
+    }
+    Link<R> u;
+    U.hop_link(mu, fwd, fwd ? e : o, fwd ? i : j, u, lsc);
+    const R k = (R)hop_sign(g, st, mu, fwd) * sc * lsc * hscale;
+    if (fwd) {
+      mul_u(u, h, f);
+      recon_fwd<R, DAG>(b, mu, f, k);
+    } else {
+      mul_ud(u, h, f);
+      recon_bwd<R, DAG>(b, mu, f, k);
+    }
+  }
+}
+
+// the sum over all directions.  b is accumulated into, so a caller either
+// zeroes it or starts it with the site-local terms of its operator.
 template <Prec PS, bool DAG, typename UV>
 __device__ __forceinline__ void wilson_hop(const Geom& g, int e, int i, const Site& st,
                                            const SpinorView<PS>& in, const UV& U,
                                            Spinor<typename SpinorView<PS>::R>& b,
                                            typename SpinorView<PS>::R hscale = 1) {
-  using R = typename SpinorView<PS>::R;
-  const int o = 1 - e;
 #pragma unroll
-  for (int mu = 3; mu >= 0; mu--) {
-    // forward hop
-    {
-      int j = neighbour(g, st, i, mu, true);
-      cx<R> h[2][3], f[2][3];
-      R sc, lsc;
-      if (mu == 3) {
-        // (1 -+ gamma_4) keeps two spins: (3,4) for d, (1,2) for d_dag
-        in.load_pair_raw(j, DAG ? 0 : 2, h, sc);
-      } else if constexpr (PS == Prec::F16) {
-        float2 F[4][3];
-        in.load_biased(j, F, sc);
-        project_biased<DAG>(F, mu, true, h);
-      } else {
-        Spinor<R> p;
-        in.load_raw(j, p, sc);
-        project<R, DAG>(p, mu, true, h);
-      }
-      Link<R> u;
-      U.hop_link(mu, true, e, i, u, lsc);
-      mul_u(u, h, f);
-      recon_fwd<R, DAG>(b, mu, f, (R)hop_sign(g, st, mu, true) * sc * lsc * hscale);
-    }
-    // backward hop
-    {
-      int j = neighbour(g, st, i, mu, false);
-      cx<R> h[2][3], f[2][3];
-      R sc, lsc;
-      if (mu == 3) {
-        in.load_pair_raw(j, DAG ? 2 : 0, h, sc);
-      } else if constexpr (PS == Prec::F16) {
-        float2 F[4][3];
-        in.load_biased(j, F, sc);
-        project_biased<DAG>(F, mu, false, h);
-      } else {
-        Spinor<R> p;
-        in.load_raw(j, p, sc);
-        project<R, DAG>(p, mu, false, h);
-      }
-      Link<R> u;
-      U.hop_link(mu, false, o, j, u, lsc);
-      mul_ud(u, h, f);
-      recon_bwd<R, DAG>(b, mu, f, (R)hop_sign(g, st, mu, false) * sc * lsc * hscale);
-    }
-  }
+  for (int mu = 3; mu >= 0; mu--) wilson_hop_mu<PS, DAG>(g, e, i, st, in, U, b, hscale, mu);
 }
 
 // wilson_hop for int16 fields with every link of the site loaded first: the

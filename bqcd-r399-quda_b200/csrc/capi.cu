@@ -259,7 +259,7 @@ int cg_core(bqcdg_ctx* c, double2* x, double2* b, const OpParams& op, Prec slopp
       if (timed) kt.end();
       launch_cg_pass4(sloppy, gs, t, q, gauge_of(c, sloppy), aee_of(c, sloppy), op, rs, c->red, c->dcg, c->stream, 1,
                       nullptr, nullptr, true, true);
-      launch_cg_step(c->red, c->dcg, 1, nblocks(gs.volh), c->stream);
+      launch_cg_step(c->red, c->dcg, 1, site_blocks(sloppy, gs), c->stream);
       launch_cg_pupdate(sloppy, g, p, rs, c->dcg, c->stream, 1, xs, CgExpect{{iter0 + k + 1}}, true);
     }
     CKL();
@@ -514,7 +514,7 @@ int cg_batch(bqcdg_ctx* c, double2** x, double2** b, int nb, const OpParams& op,
                           c->stream, nb, dkap, AlphaFin{c->red.partial, c->red.maxblocks, c->dcg}, true);
         launch_cg_pass4(sloppy, g, B.t, B.q, gauge_of(c, sloppy), aee_of(c, sloppy), op, B.rs, c->red, c->dcg,
                         c->stream, nb, drho, dkap, true, true);
-        launch_cg_step(c->red, c->dcg, nb, nblocks(g.volh), c->stream);
+        launch_cg_step(c->red, c->dcg, nb, dkap ? nblocks(g.volh) : site_blocks(sloppy, g), c->stream);
       }
       launch_cg_pupdate(sloppy, g, B.p, B.rs, c->dcg, c->stream, nb, B.xs, expect, true);
     }

@@ -215,6 +215,10 @@ __global__ void __launch_bounds__(kBlock, Occ<P>::min_blocks) k_pass1(Geom g, Sp
 void launch_mtil_pass1(Prec p, const Geom& g, bool dag, SpinorPtr out_o, SpinorPtr in_e, const void* gauge,
                        CloverPtr ainv_oo, const OpParams& op, const CgScalars* cg, cudaStream_t s, int nr,
                        const double* kappa_rhs, AlphaFin fin, bool chain) {
+  if (split_sites(p, g) && !kappa_rhs) {
+    launch_split_pass1(g, dag, out_o, in_e, gauge, ainv_oo, op, cg, s, nr, fin, chain);
+    return;
+  }
   dim3 grid((nblocks(g.volh) + (fin.partial ? 1 : 0)) * nr);
   int hc = op.csw_kappa != 0.0;
   double hv = dag ? op.h : -op.h;
@@ -348,6 +352,10 @@ void launch_mtil_pass2(Prec p, const Geom& g, bool dag, SpinorPtr out_e, SpinorP
   double hv = dag ? -op.h : op.h;
   bool reduce = norm_out != nullptr || cg != nullptr;
   defer_alpha = defer_alpha && cg && !norm_out;  // only alpha can wait for the next pass
+  if (split_sites(p, g) && !kappa_rhs && (defer_alpha || !reduce)) {
+    launch_split_pass2(g, dag, out_e, t_o, in_e, gauge, a_ee, op, red, reduce, cg, s, nr, rho_rhs, chain);
+    return;
+  }
 #define P2(PP, D, RR, K)                                                                                        \
   launch_chain(chain, k_pass2<PP, D, RR, K>, grid, kBlock, s, g, out_e, t_o, in_e, gauge, a_ee, hc, bcoef, hv,  \
                op.rho, red, norm_out, cg, nr, rho_rhs, op.kappa, kappa_rhs, defer_alpha)
@@ -451,6 +459,10 @@ void launch_cg_step(RedScratch red, CgScalars* cg, int nr, int nsb, cudaStream_t
 void launch_cg_pass4(Prec p, const Geom& g, SpinorPtr t_o, SpinorPtr q_e, const void* gauge, CloverPtr a_ee,
                      const OpParams& op, SpinorPtr r, RedScratch red, CgScalars* cg, cudaStream_t s, int nr,
                      const double* rho_rhs, const double* kappa_rhs, bool defer_step, bool chain) {
+  if (split_sites(p, g) && !kappa_rhs && defer_step) {
+    launch_split_pass4(g, t_o, q_e, gauge, a_ee, op, r, red, cg, s, nr, rho_rhs, chain);
+    return;
+  }
   dim3 grid(nblocks(g.volh) * nr);
   int hc = op.csw_kappa != 0.0;
   double bcoef = -op.kappa * op.kappa / (1.0 + op.h * op.h);

@@ -158,6 +158,20 @@ void launch_mtil_pass2_n(Prec p, const Geom& g, SpinorPtr out_e, SpinorPtr t_o, 
 void launch_cg_pass4_n(Prec p, const Geom& g, SpinorPtr t_o, SpinorPtr q_e, const void* gauge, CloverPtr a_ee,
                        const OpParams& op, SpinorPtr r, RedScratch red, CgScalars* cg, cudaStream_t s, int nr,
                        const double* rho_rhs, int nbt, bool defer_step = false, bool chain = false);
+// the same three passes of FP64 fields with four threads per site
+// (dslash_split.cu), which the launchers above take where split_sites says so:
+// stored clover blocks, one kappa, deferred sums.  site_blocks: the block
+// partials of a pass, at most kRedVals maxblocks per right-hand side
+bool split_sites(Prec p, const Geom& g);
+int site_blocks(Prec p, const Geom& g);
+void launch_split_pass1(const Geom& g, bool dag, SpinorPtr out, SpinorPtr in, const void* gauge, CloverPtr a,
+                        const OpParams& op, const CgScalars* cg, cudaStream_t s, int nr, AlphaFin fin, bool chain);
+void launch_split_pass2(const Geom& g, bool dag, SpinorPtr out, SpinorPtr t, SpinorPtr x, const void* gauge,
+                        CloverPtr a, const OpParams& op, RedScratch red, bool sum, const CgScalars* cg,
+                        cudaStream_t s, int nr, const double* rho_rhs, bool chain);
+void launch_split_pass4(const Geom& g, SpinorPtr t, SpinorPtr q, const void* gauge, CloverPtr a, const OpParams& op,
+                        SpinorPtr r, RedScratch red, const CgScalars* cg, cudaStream_t s, int nr,
+                        const double* rho_rhs, bool chain);
 // p = r + beta p, and the x += alpha p of iteration expect.n[rhs] if that
 // iteration ran
 void launch_cg_pupdate(Prec p, const Geom& g, SpinorPtr pvec, SpinorPtr r, CgScalars* cg, cudaStream_t s,
