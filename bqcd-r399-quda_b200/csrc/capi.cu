@@ -236,31 +236,43 @@ int cg_core(bqcdg_ctx* c, double2* x, double2* b, const OpParams& op, Prec slopp
 
   int batch = 4;
   const Geom& gs = geom_of(c, sloppy);  // stencil geometry (12-real FP64 links when SU(3))
+  const int nsb = site_blocks(sloppy, gs);  // block partials of a pass
+  const bool fused = nsb <= kFusedStep;
   while (!h.done) {
-    nl += 6 * batch;
+    nl += (fused ? 5 : 6) * batch;
     const int iter0 = h.iter;
     for (int k = 0; k < batch; k++) {
       // pass 1, pass 2 (+|M~p|^2 partials), pass 3 (+ their sum -> alpha), pass 4 (+x,r update, |r|^2
-      // partials), the CG step, p update.  With time_kernels, passes 1 and 3 of the second iteration of
+      // partials), the CG step, p and x update.  With time_kernels, passes 1 and 3 of the second iteration of
       // each batch are bracketed by events: a sample of every batch in the steady state (the first
       // iteration follows the host's read of the scalars, or a reliable update whose FP64 fields have
       // displaced the int16 ones from L2), and events between all launches would lengthen the solve
       // they time.
       const bool timed = k == 1;
+      // the fused update leaves the stepped scalars in the other of two slots;
+      // a batch is even, so it ends in slot 0
+      CgScalars *cg = c->dcg + (fused ? k & 1 : 0), *next = c->dcg + (~k & 1);
+      // what pass 1 may read before its wait: the slot that the launch before
+      // it does not write (it then runs once in vain when the solve stops)
+      const CgScalars* prev = fused && k > 0 ? next : cg;
       if (timed) kt.begin();
-      launch_mtil_pass1(sloppy, gs, false, t, p, gauge_of(c, sloppy), ainv_of(c, sloppy), op, c->dcg, c->stream, 1,
+      launch_mtil_pass1(sloppy, gs, false, t, p, gauge_of(c, sloppy), ainv_of(c, sloppy), op, prev, c->stream, 1,
                         nullptr, AlphaFin{}, true);
       if (timed) kt.end();
       launch_mtil_pass2(sloppy, gs, false, q, t, p, gauge_of(c, sloppy), aee_of(c, sloppy), op, c->red, nullptr,
-                        c->dcg, c->stream, 1, nullptr, nullptr, true, true);
+                        cg, c->stream, 1, nullptr, nullptr, true, true);
       if (timed) kt.begin();
-      launch_mtil_pass1(sloppy, gs, true, t, q, gauge_of(c, sloppy), ainv_of(c, sloppy), op, c->dcg, c->stream, 1,
-                        nullptr, AlphaFin{c->red.partial, c->red.maxblocks, c->dcg}, true);
+      launch_mtil_pass1(sloppy, gs, true, t, q, gauge_of(c, sloppy), ainv_of(c, sloppy), op, cg, c->stream, 1,
+                        nullptr, AlphaFin{c->red.partial, c->red.maxblocks, cg}, true);
       if (timed) kt.end();
-      launch_cg_pass4(sloppy, gs, t, q, gauge_of(c, sloppy), aee_of(c, sloppy), op, rs, c->red, c->dcg, c->stream, 1,
+      launch_cg_pass4(sloppy, gs, t, q, gauge_of(c, sloppy), aee_of(c, sloppy), op, rs, c->red, cg, c->stream, 1,
                       nullptr, nullptr, true, true);
-      launch_cg_step(c->red, c->dcg, 1, site_blocks(sloppy, gs), c->stream);
-      launch_cg_pupdate(sloppy, g, p, rs, c->dcg, c->stream, 1, xs, CgExpect{{iter0 + k + 1}}, true);
+      if (fused) {
+        launch_cg_update(sloppy, g, p, rs, xs, cg, next, c->red, nsb, c->stream);
+      } else {
+        launch_cg_step(c->red, cg, 1, nsb, c->stream);
+        launch_cg_pupdate(sloppy, g, p, rs, cg, c->stream, 1, xs, CgExpect{{iter0 + k + 1}}, true);
+      }
     }
     CKL();
     int st = read_cg(c);

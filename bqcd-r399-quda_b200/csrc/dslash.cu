@@ -533,4 +533,62 @@ void launch_cg_pupdate(Prec p, const Geom& g, SpinorPtr pvec, SpinorPtr r, CgSca
 #undef PU
 }
 
+// k_cg_step and k_cg_pupdate in one launch, for one right-hand side: every CTA
+// sums the |r|^2 partials of the launch before and takes the scalar step for
+// itself, CTA 0 stores it.  It goes to `next`, which the following iteration
+// reads, since other CTAs still read `cur`.
+template <Prec P, Prec RP>
+__global__ void __launch_bounds__(kBlock, P == Prec::F64 ? 3 : 5) k_cg_update(Geom g, SpinorPtr pp, SpinorPtr rp, SpinorPtr xp,
+                                                      const CgScalars* cur, CgScalars* next, RedScratch red, int nsb) {
+  using R = typename SpinorView<P>::R;
+  using RR = typename SpinorView<RP>::R;
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  const bool first = i == 0, live = i < g.volh;
+  if (cur->done) {  // this iteration did not run
+    chain_wait();
+    if (first) *next = *cur;
+    return;
+  }
+  auto pv = sview<P>(pp, g.stride);
+  auto xv = sview<RP>(xp, g.stride);
+  Spinor<R> pl;
+  R psc;
+  Spinor<RR> xl, rl;
+  if (live) {
+    pv.load_raw(i, pl, psc);
+    xv.load(i, xl);
+  }
+  CgScalars c = *cur;
+  chain_wait();
+  if (live) after_wait(sview<RP>(rp, g.stride)).load(i, rl);
+  double tot[1];
+  final_sum<1>(after_wait(red.partial), red.maxblocks, nsb, tot);
+  cg_scalar_step(&c, tot[0]);
+  if (first) *next = c;
+  if (!live) return;
+  const RR a = (RR)c.alpha * (RR)psc;
+#pragma unroll
+  for (int s = 0; s < 4; s++)
+#pragma unroll
+    for (int k = 0; k < 3; k++) xl.c[s][k] = xl.c[s][k] + a * mkc((RR)pl.c[s][k].x, (RR)pl.c[s][k].y);
+  xv.store(i, xl);
+  if (c.done) return;
+  const R b = (R)c.beta * psc;
+#pragma unroll
+  for (int s = 0; s < 4; s++)
+#pragma unroll
+    for (int k = 0; k < 3; k++) pl.c[s][k] = mkc((R)rl.c[s][k].x, (R)rl.c[s][k].y) + b * pl.c[s][k];
+  pv.store(i, pl);
+}
+
+void launch_cg_update(Prec p, const Geom& g, SpinorPtr pvec, SpinorPtr r, SpinorPtr x, const CgScalars* cur,
+                      CgScalars* next, RedScratch red, int nsb, cudaStream_t s) {
+  dim3 grid(nblocks(g.volh));
+#define CU(PP, RR) launch_chain(true, k_cg_update<PP, RR>, grid, kBlock, s, g, pvec, r, x, cur, next, red, nsb)
+  if (p == Prec::F64) CU(Prec::F64, Prec::F64);
+  else if (p == Prec::F32) CU(Prec::F32, Prec::F32);
+  else CU(Prec::F16, Prec::F32);
+#undef CU
+}
+
 }  // namespace bqcdg

@@ -177,6 +177,15 @@ void launch_split_pass4(const Geom& g, SpinorPtr t, SpinorPtr q, const void* gau
 void launch_cg_pupdate(Prec p, const Geom& g, SpinorPtr pvec, SpinorPtr r, CgScalars* cg, cudaStream_t s,
                        int nr, SpinorPtr x, const CgExpect& expect, bool chain = false);
 
+// both, for one right-hand side and up to kFusedStep block partials: every CTA
+// sums them itself.  The stepped scalars go to `next`; when the iteration did
+// not run they are those of `cur`.  At 60 partials a mixed solve (10x6x14x18)
+// takes 4.4 instead of 4.7 ms and FP64 CG at 8^4 3.8 instead of 4.0 ms; at 512
+// and 945 the sums cost what the launch saves (12.9, 6.9 ms -> 13.0, 7.0 ms).
+constexpr int kFusedStep = 2 * kBlock;
+void launch_cg_update(Prec p, const Geom& g, SpinorPtr pvec, SpinorPtr r, SpinorPtr x, const CgScalars* cur,
+                      CgScalars* next, RedScratch red, int nsb, cudaStream_t s);
+
 // ---- block solver (blockcg.cu) ----
 // out[i * s + j] = <a_i, b_j> (FP64) for two blocks of s <= 16 FP32 fields
 // (batched layout); partial: block_gram_scratch_pairs() complex doubles
