@@ -1085,7 +1085,8 @@ __device__ __forceinline__ void wilson_hop(const Geom& g, int e, int i, const Si
 // they stream from HBM while the gathers, which mostly hit L2, proceed hop by
 // hop.  Same products in the same order as wilson_hop, so the result is
 // bit-identical; it needs about 40 more registers.
-template <bool DAG>
+// WAIT: the gathered field is written by the launch before (chain_wait).
+template <bool DAG, bool WAIT = true>
 __device__ __forceinline__ void wilson_hop_lf(const Geom& g, int e, int i, const Site& st,
                                               const SpinorView<Prec::F16>& in0, const GaugeView<Prec::F16>& U,
                                               Spinor<float>& b, float hscale = 1.f) {
@@ -1104,8 +1105,11 @@ __device__ __forceinline__ void wilson_hop_lf(const Geom& g, int e, int i, const
       W[mu][1][w] = ld_once(ub + (size_t)((mu * 2 + o) * 3 + w) * S + J[mu][1]);
     }
   }
-  chain_wait();  // the links do not depend on the launch before
-  const SpinorView<Prec::F16> in = after_wait(in0);
+  SpinorView<Prec::F16> in = in0;
+  if constexpr (WAIT) {
+    chain_wait();  // the links do not depend on the launch before
+    in = after_wait(in0);
+  }
 #pragma unroll
   for (int mu = 3; mu >= 0; mu--) {
 #pragma unroll

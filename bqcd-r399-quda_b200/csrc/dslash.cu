@@ -241,7 +241,7 @@ void launch_mtil_pass1(Prec p, const Geom& g, bool dag, SpinorPtr out_o, SpinorP
 // they come before chain_wait); b is applied inside the hop sum and the storage
 // scales of x and A_ee as one factor, so no field is rescaled component by
 // component.
-template <Prec P, bool DAG, bool KT>
+template <Prec P, bool DAG, bool KT, bool LATE>
 __device__ __forceinline__ void pass2_core(const Geom& g, int i, const SpinorView<P>& t, const SpinorView<P>& xin,
                                            const GaugeView<P>& U, const CloverPtr& aee, int has_clover, double bcoef,
                                            double hval, double rho, Spinor<typename SpinorView<P>::R>& out,
@@ -279,14 +279,26 @@ __device__ __forceinline__ void pass2_core(const Geom& g, int i, const SpinorVie
   }
   const Site st = site_coords(g, i, 0);
   if constexpr (P == Prec::F16) {
-    wilson_hop_lf<DAG>(g, 0, i, st, t, U, out, (R)bcoef);  // waits (chain_wait) once its links are requested
+    wilson_hop_lf<DAG, LATE>(g, 0, i, st, t, U, out, (R)bcoef);  // LATE: waits once its links are requested
   } else {
-    chain_wait();
-    wilson_hop<P, DAG>(g, 0, i, st, after_wait(t), U, out, (R)bcoef);
+    if constexpr (LATE) chain_wait();
+    wilson_hop<P, DAG>(g, 0, i, st, LATE ? after_wait(t) : t, U, out, (R)bcoef);
   }
 }
 
-template <Prec P, bool DAG, bool REDUCE, bool KT>
+// Where a second pass waits (chain_wait).  LATE: with its local terms done and
+// its links requested, which shortens a launch of few CTAs.  But nothing can
+// be moved across the wait, and an int16 pass of many waves, which hides its
+// latencies behind other CTAs, pays for that: at 32^3x64 k_pass2 takes 109
+// instead of 104 us and k_cg_pass4 117 instead of 112 us, so those wait first.
+// The solve: 246.7 -> 244.4 ms.  At 16^3x32 (512 CTAs, one wave) the early wait
+// costs a mixed solve 7 %, and the passes that form A(kappa) gain nothing from
+// it (8 systems at 16^3x32: 80.6 ms late, 81.1 ms early).
+inline bool late_wait(Prec p, const Geom& g, int nr) {
+  return p != Prec::F16 || g.clover_t || nblocks(g.volh) * nr <= 148 * 4 * 3;
+}
+
+template <Prec P, bool DAG, bool REDUCE, bool KT, bool LATE>
 __global__ void __launch_bounds__(kBlock, Occ<P>::min_blocks2) k_pass2(Geom g, SpinorPtr outp, SpinorPtr tp, SpinorPtr xp,
                                                   const void* gauge, CloverPtr aee, int has_clover, double bcoef,
                                                   double hval, double rho, RedScratch red, double* norm_out,
@@ -298,6 +310,7 @@ __global__ void __launch_bounds__(kBlock, Occ<P>::min_blocks2) k_pass2(Geom g, S
     chain_wait();
     return;
   }
+  if constexpr (!LATE) chain_wait();
   if (rho_rhs) rho = rho_rhs[tl.rhs];   // a shift per right-hand side
   if (kappa_rhs) {                       // a hopping parameter per right-hand side
     kappa = kappa_rhs[tl.rhs];
@@ -307,11 +320,12 @@ __global__ void __launch_bounds__(kBlock, Occ<P>::min_blocks2) k_pass2(Geom g, S
   double acc[1] = {0.0};
   if (i < g.volh) {
     auto t = sview<P>(rhs_of(tp, tl.rhs), g.stride);
+    if constexpr (!LATE) t = after_wait(t);
     auto xin = sview<P>(rhs_of(xp, tl.rhs), g.stride);
     auto out = sview<P>(rhs_of(outp, tl.rhs), g.stride);
     auto U = gview<P>(gauge, g);
     Spinor<R> o;
-    pass2_core<P, DAG, KT>(g, i, t, xin, U, aee, has_clover, bcoef, hval, rho, o, kappa);
+    pass2_core<P, DAG, KT, LATE>(g, i, t, xin, U, aee, has_clover, bcoef, hval, rho, o, kappa);
     out.store(i, o);
     if (REDUCE) {
 #pragma unroll
@@ -319,7 +333,7 @@ __global__ void __launch_bounds__(kBlock, Occ<P>::min_blocks2) k_pass2(Geom g, S
 #pragma unroll
         for (int c = 0; c < 3; c++) acc[0] += (double)norm2(o.c[s][c]);
     }
-  } else {
+  } else if (LATE) {
     chain_wait();
   }
   if (REDUCE) {
@@ -356,20 +370,24 @@ void launch_mtil_pass2(Prec p, const Geom& g, bool dag, SpinorPtr out_e, SpinorP
     launch_split_pass2(g, dag, out_e, t_o, in_e, gauge, a_ee, op, red, reduce, cg, s, nr, rho_rhs, chain);
     return;
   }
-#define P2(PP, D, RR, K)                                                                                        \
-  launch_chain(chain, k_pass2<PP, D, RR, K>, grid, kBlock, s, g, out_e, t_o, in_e, gauge, a_ee, hc, bcoef, hv,  \
+  const bool late = late_wait(p, g, nr);
+#define P2L(PP, D, RR, K, LT)                                                                                       \
+  launch_chain(chain, k_pass2<PP, D, RR, K, LT>, grid, kBlock, s, g, out_e, t_o, in_e, gauge, a_ee, hc, bcoef, hv, \
                op.rho, red, norm_out, cg, nr, rho_rhs, op.kappa, kappa_rhs, defer_alpha)
+#define P2(PP, D, RR, K) \
+  if (late) P2L(PP, D, RR, K, true); else P2L(PP, D, RR, K, (PP != Prec::F16))
 #define P2R(PP, D)                                         \
   if (g.clover_t) {                                        \
-    if (reduce) P2(PP, D, true, true); else P2(PP, D, false, true);   \
+    if (reduce) { P2(PP, D, true, true); } else { P2(PP, D, false, true); }   \
   } else {                                                 \
-    if (reduce) P2(PP, D, true, false); else P2(PP, D, false, false); \
+    if (reduce) { P2(PP, D, true, false); } else { P2(PP, D, false, false); } \
   }
   if (p == Prec::F64) { if (dag) { P2R(Prec::F64, true) } else { P2R(Prec::F64, false) } }
   else if (p == Prec::F32) { if (dag) { P2R(Prec::F32, true) } else { P2R(Prec::F32, false) } }
   else { if (dag) { P2R(Prec::F16, true) } else { P2R(Prec::F16, false) } }
 #undef P2R
 #undef P2
+#undef P2L
 }
 
 // ---------------------------------------------------------------------------
@@ -386,7 +404,7 @@ struct XR<Prec::F32> {
   using View = SpinorView<Prec::F32>;
 };
 
-template <Prec P, Prec XP, bool KT>
+template <Prec P, Prec XP, bool KT, bool LATE>
 __global__ void __launch_bounds__(kBlock, Occ<P>::min_blocks2) k_cg_pass4(Geom g, SpinorPtr tp, SpinorPtr qp, const void* gauge,
                                                      CloverPtr aee, int has_clover, double bcoef, double hval,
                                                      double rho, SpinorPtr rp,
@@ -400,6 +418,7 @@ __global__ void __launch_bounds__(kBlock, Occ<P>::min_blocks2) k_cg_pass4(Geom g
     chain_wait();
     return;
   }
+  if constexpr (!LATE) chain_wait();
   if (rho_rhs) rho = rho_rhs[tl.rhs];  // a shift per right-hand side
   if (kappa_rhs) {                      // a hopping parameter per right-hand side
     kappa = kappa_rhs[tl.rhs];
@@ -409,11 +428,12 @@ __global__ void __launch_bounds__(kBlock, Occ<P>::min_blocks2) k_cg_pass4(Geom g
   double acc[1] = {0.0};
   if (i < g.volh) {
     auto t = sview<P>(rhs_of(tp, tl.rhs), g.stride);
+    if constexpr (!LATE) t = after_wait(t);
     auto q = sview<P>(rhs_of(qp, tl.rhs), g.stride);
     auto U = gview<P>(gauge, g);
     auto rv = sview<XP>(rhs_of(rp, tl.rhs), g.stride);
     Spinor<R> ap;
-    pass2_core<P, true, KT>(g, i, t, q, U, aee, has_clover, bcoef, hval, rho, ap, kappa);
+    pass2_core<P, true, KT, LATE>(g, i, t, q, U, aee, has_clover, bcoef, hval, rho, ap, kappa);
     const RX a = (RX)cg->alpha;  // set by the launch before
     Spinor<RX> rl;
     rv.load(i, rl);
@@ -425,7 +445,7 @@ __global__ void __launch_bounds__(kBlock, Occ<P>::min_blocks2) k_cg_pass4(Geom g
         acc[0] += (double)norm2(rl.c[s][c]);
       }
     rv.store(i, rl);
-  } else {
+  } else if (LATE) {
     chain_wait();
   }
   double* part = red.partial + (size_t)tl.rhs * kRedVals * red.maxblocks;
@@ -467,15 +487,19 @@ void launch_cg_pass4(Prec p, const Geom& g, SpinorPtr t_o, SpinorPtr q_e, const 
   int hc = op.csw_kappa != 0.0;
   double bcoef = -op.kappa * op.kappa / (1.0 + op.h * op.h);
   double hv = -op.h;  // mtil_dag
-#define P4(PP, XX, K)                                                                                         \
-  launch_chain(chain, k_cg_pass4<PP, XX, K>, grid, kBlock, s, g, t_o, q_e, gauge, a_ee, hc, bcoef, hv, op.rho, r, \
-               red, cg, nr, rho_rhs, op.kappa, kappa_rhs, defer_step)
-#define P4K(PP, XX) if (g.clover_t) P4(PP, XX, true); else P4(PP, XX, false);
+  const bool late = late_wait(p, g, nr);
+#define P4L(PP, XX, K, LT)                                                                                     \
+  launch_chain(chain, k_cg_pass4<PP, XX, K, LT>, grid, kBlock, s, g, t_o, q_e, gauge, a_ee, hc, bcoef, hv, op.rho, \
+               r, red, cg, nr, rho_rhs, op.kappa, kappa_rhs, defer_step)
+#define P4(PP, XX, K) \
+  if (late) P4L(PP, XX, K, true); else P4L(PP, XX, K, (PP != Prec::F16))
+#define P4K(PP, XX) if (g.clover_t) { P4(PP, XX, true); } else { P4(PP, XX, false); }
   if (p == Prec::F64) { P4K(Prec::F64, Prec::F64) }
   else if (p == Prec::F32) { P4K(Prec::F32, Prec::F32) }
   else { P4K(Prec::F16, Prec::F32) }
 #undef P4K
 #undef P4
+#undef P4L
 }
 
 // p = r + beta p   (sc_xpby, cg.F90:116) and the x += alpha p of the same
