@@ -287,12 +287,12 @@ int cg_core(bqcdg_ctx* c, double2* x, double2* b, const OpParams& op, Prec slopp
     }
     // reliable update: x += x_s, r = b - A x in FP64
     const bool periodic = !(h.rtr < h.delta2 * h.maxr2);
-    nl += 7;
+    nl += 6;
     launch_accum_x(g, x, (float4*)xs.v, c->stream);
     apply_mdagm(c, Prec::F64, S(ax), S(x), S(t64), S(q64), op);
-    launch_residual(g, r, b, ax, Prec::F32, rs, c->red, c->dres, c->stream);
+    launch_update_residual(g, rs, b, ax, sloppy, p, c->red, c->dres, c->stream);
     CKL();
-    CK(cudaMemcpyAsync(c->hres, c->dres, 2 * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
+    CK(cudaMemcpyAsync(c->hres, c->dres, 3 * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
     CK(cudaStreamSynchronize(c->stream));
     ru++;
     double rtrue = c->hres[0];
@@ -307,11 +307,7 @@ int cg_core(bqcdg_ctx* c, double2* x, double2* b, const OpParams& op, Prec slopp
     if (sloppy == Prec::F16 && forced >= 2) { h.rtr = rtrue; stalled = true; break; }
     // continue from the true residual with p re-orthogonalised against it:
     // p = r + beta (p - (<r,p>/|r|^2) r), beta = |r|^2 / |r_old|^2
-    launch_rdot(g, rs, sloppy, p, c->red, c->dres, c->stream);
-    CKL();
-    CK(cudaMemcpyAsync(c->hres, c->dres, sizeof(double), cudaMemcpyDeviceToHost, c->stream));
-    CK(cudaStreamSynchronize(c->stream));
-    double rpc = c->hres[0] / rtrue;
+    double rpc = c->hres[2] / rtrue;
     h.beta = rtrue / h.rtr_old;
     h.rtr = rtrue;
     h.maxr2 = rtrue;
@@ -319,7 +315,7 @@ int cg_core(bqcdg_ctx* c, double2* x, double2* b, const OpParams& op, Prec slopp
     h.done = 0;
     { int st_ = write_cg(c); if (st_) return st_; }
     launch_p_reorth(g, sloppy, p, rs, rpc, h.beta, c->stream);
-    nl += 2;
+    nl += 1;
     CKL();
   }
   CK(cudaEventRecord(c->ev1, c->stream));
@@ -417,17 +413,21 @@ int ensure_batch(bqcdg_ctx* c, Prec p, int nb) {
   return BQCDG_OK;
 }
 
-// r = b - A x in FP64 for one right-hand side, r copied into rs (F32);
-// returns |r|^2 and |b|^2
-int fp64_residual(bqcdg_ctx* c, double2* x, double2* b, const OpParams& op, SpinorPtr rs, double* r2, double* b2) {
-  double2 *r = c->sp64(0), *ax = c->sp64(1);
-  apply_mdagm(c, Prec::F64, S(ax), S(x), S(c->sp64(2)), S(c->sp64(3)), op);
-  launch_residual(c->g, r, b, ax, Prec::F32, rs, c->red, c->dres, c->stream);
+// queues r = b - A x in FP64 for right-hand side k of a batch: r goes to rs
+// (FP32), {|r|^2, |b|^2, <r, p>} to slot k of dres
+int queue_residual(bqcdg_ctx* c, int k, double2* x, double2* b, const OpParams& op, Prec sloppy, SpinorPtr rs,
+                   SpinorPtr p) {
+  double2 *ax = c->sp64(1), *t = c->sp64(2), *q = c->sp64(3);
+  if (!ax || !t || !q) return BQCDG_ENOMEM;
+  apply_mdagm(c, Prec::F64, S(ax), S(x), S(t), S(q), op);
+  launch_update_residual(c->g, rs, b, ax, sloppy, p, c->red, c->dres + 3 * k, c->stream);
+  return BQCDG_OK;
+}
+// the slots of nb right-hand sides, once the queued residuals are there
+int read_residuals(bqcdg_ctx* c, int nb) {
   CKL();
-  CK(cudaMemcpyAsync(c->hres, c->dres, 2 * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
+  CK(cudaMemcpyAsync(c->hres, c->dres, 3 * nb * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
   CK(cudaStreamSynchronize(c->stream));
-  *r2 = c->hres[0];
-  if (b2) *b2 = c->hres[1];
   return BQCDG_OK;
 }
 
@@ -474,9 +474,11 @@ int cg_batch(bqcdg_ctx* c, double2** x, double2** b, int nb, const OpParams& op,
   CK(cudaEventRecord(c->ev0, c->stream));
   std::vector<int> ru(nb, 0), fin(nb, 0), conv(nb, 0), nl(nb, 0), stall(nb, 0), stalled(nb, 0);
   std::vector<double> best(nb, 0.0);
+  for (int k = 0; k < nb; k++)
+    if ((st = queue_residual(c, k, x[k], b[k], ops[k], sloppy, rhs_of(B.rs, k), rhs_of(B.p, k)))) return st;
+  if ((st = read_residuals(c, nb))) return st;
   for (int k = 0; k < nb; k++) {
-    double r2, b2;
-    if ((st = fp64_residual(c, x[k], b[k], ops[k], rhs_of(B.rs, k), &r2, &b2))) return st;
+    const double r2 = c->hres[3 * k];
     launch_spinor_convert(g, sloppy, rhs_of(B.p, k), Prec::F32, rhs_of(B.rs, k), c->stream);
     launch_zero(g, Prec::F32, rhs_of(B.xs, k), c->stream);
     CKL();
@@ -490,7 +492,7 @@ int cg_batch(bqcdg_ctx* c, double2** x, double2** b, int nb, const OpParams& op,
     h.ru_every = kRuEvery;
     h.last_ru = 0;
     best[k] = r2;
-    info[k].b2 = b2;
+    info[k].b2 = c->hres[3 * k + 1];
     if (!(r2 == r2)) { h.done = 4; fin[k] = 1; }
     else if (r2 <= stop[k]) { h.done = 1; fin[k] = 1; conv[k] = 1; }
     else if (maxiter <= 0) { h.done = 3; fin[k] = 1; }
@@ -535,17 +537,22 @@ int cg_batch(bqcdg_ctx* c, double2** x, double2** b, int nb, const OpParams& op,
     CK(cudaMemcpyAsync(c->hcg, c->dcg, sizeof(CgScalars) * nb, cudaMemcpyDeviceToHost, c->stream));
     CK(cudaStreamSynchronize(c->stream));
     if (batch < 16) batch *= 2;
-    std::vector<int> resume;
+    std::vector<int> update, resume;
     for (int k = 0; k < nb; k++) {
       CgScalars& h = c->hcg[k];
       if (fin[k] || h.done == 0) continue;
       if (h.done == 4) { fin[k] = 1; continue; }
       // reliable update of right-hand side k: x += x_s, r = b - A x in FP64
       launch_accum_x(g, x[k], (float4*)rhs_of(B.xs, k).v, c->stream);
-      double rt;
-      if ((st = fp64_residual(c, x[k], b[k], ops[k], rhs_of(B.rs, k), &rt, nullptr))) return st;
+      if ((st = queue_residual(c, k, x[k], b[k], ops[k], sloppy, rhs_of(B.rs, k), rhs_of(B.p, k)))) return st;
+      update.push_back(k);
       ru[k]++;
-      launches += 7;
+      launches += 6;
+    }
+    if (!update.empty() && (st = read_residuals(c, nb))) return st;
+    for (int k : update) {
+      CgScalars& h = c->hcg[k];
+      const double rt = c->hres[3 * k];
       if (!(rt == rt)) { h.done = 4; fin[k] = 1; continue; }
       if (rt <= stop[k]) { h.rtr = rt; h.done = 1; fin[k] = 1; conv[k] = 1; continue; }
       if (h.done == 3) { h.rtr = rt; fin[k] = 1; continue; }
@@ -568,13 +575,9 @@ int cg_batch(bqcdg_ctx* c, double2** x, double2** b, int nb, const OpParams& op,
     CK(cudaMemcpyAsync(c->dcg, c->hcg, sizeof(CgScalars) * nb, cudaMemcpyHostToDevice, c->stream));
     for (int k : resume) {
       // p = r + beta (p - (<r,p>/|r|^2) r)
-      launch_rdot(g, rhs_of(B.rs, k), sloppy, rhs_of(B.p, k), c->red, c->dres, c->stream);
-      CKL();
-      CK(cudaMemcpyAsync(c->hres, c->dres, sizeof(double), cudaMemcpyDeviceToHost, c->stream));
-      CK(cudaStreamSynchronize(c->stream));
-      launch_p_reorth(g, sloppy, rhs_of(B.p, k), rhs_of(B.rs, k), c->hres[0] / c->hcg[k].rtr, c->hcg[k].beta,
-                      c->stream);
-      launches += 2;
+      launch_p_reorth(g, sloppy, rhs_of(B.p, k), rhs_of(B.rs, k), c->hres[3 * k + 2] / c->hcg[k].rtr,
+                      c->hcg[k].beta, c->stream);
+      launches += 1;
     }
     CKL();
   }
@@ -781,11 +784,11 @@ int bqcdg_create(bqcdg_ctx** out, const int L[4], const int bc[4], int device) {
     e = c->alloc((void**)&c->red.partial, sizeof(double) * kRedVals * kMaxRhs * c->red.maxblocks);
   if (e == cudaSuccess) e = c->alloc((void**)&c->red.counter, sizeof(unsigned int) * kMaxRhs);
   if (e == cudaSuccess) e = cudaMemsetAsync(c->red.counter, 0, sizeof(unsigned int) * kMaxRhs, c->stream);
-  if (e == cudaSuccess) e = c->alloc((void**)&c->dres, sizeof(double) * 16);
+  if (e == cudaSuccess) e = c->alloc((void**)&c->dres, sizeof(double) * 3 * kMaxRhs);
   if (e == cudaSuccess) e = c->alloc((void**)&c->drho, sizeof(double) * kMaxRhs);
   if (e == cudaSuccess) e = c->alloc((void**)&c->dkappa, sizeof(double) * kMaxRhs);
   if (e == cudaSuccess) e = c->alloc((void**)&c->dcg, sizeof(CgScalars) * kMaxRhs);
-  if (e == cudaSuccess) e = cudaMallocHost((void**)&c->hres, sizeof(double) * 16);
+  if (e == cudaSuccess) e = cudaMallocHost((void**)&c->hres, sizeof(double) * 3 * kMaxRhs);
   if (e == cudaSuccess) e = cudaMallocHost((void**)&c->hcg, sizeof(CgScalars) * kMaxRhs);
   if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
   if (e != cudaSuccess) {

@@ -56,7 +56,7 @@ struct bqcdg_ctx {
   std::vector<SpinorPtr> s32, s16;
 
   RedScratch red{};
-  double* dres = nullptr;        // device result scalars [16]
+  double* dres = nullptr;        // device result scalars [3 * kMaxRhs]
   double* hres = nullptr;        // pinned mirror
   double* drho = nullptr;        // per right-hand-side shifts of a batch [kMaxRhs]
   double* dkappa = nullptr;      // per right-hand-side hopping parameters of a batch [kMaxRhs]

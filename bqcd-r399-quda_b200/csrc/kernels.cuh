@@ -214,6 +214,9 @@ void launch_residual(const Geom& g, double2* r, const double2* b, const double2*
                      RedScratch red, double* res2, cudaStream_t s);
 // reliable-update helpers: *out = <r32, p> (real), then p = r + beta (p - rpc r)
 void launch_rdot(const Geom& g, SpinorPtr r32, Prec pp, SpinorPtr p, RedScratch red, double* out, cudaStream_t s);
+// r = b - Ax in FP32, res3 = {|r|^2, |b|^2, <r, p>} for a sloppy direction p
+void launch_update_residual(const Geom& g, SpinorPtr r32, const double2* b, const double2* ax, Prec pp, SpinorPtr p,
+                            RedScratch red, double* res3, cudaStream_t s);
 void launch_p_reorth(const Geom& g, Prec pp, SpinorPtr p, SpinorPtr r32, double rpc, double beta, cudaStream_t s);
 // x = (1 + i h gamma_5) x (h_mult_b, h_mult.F90:51-82), F64
 void launch_h_mult_b(const Geom& g, double2* x, double h, cudaStream_t s);
