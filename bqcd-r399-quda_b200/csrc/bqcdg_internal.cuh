@@ -186,11 +186,15 @@ __host__ __device__ __forceinline__ int hop_sign(const Geom& g, const Site& s, i
 // ---------------------------------------------------------------------------
 // chained launches (launch_chain): the CTAs of a launch may start while the
 // kernel before it in the stream drains.  chain_wait() returns once that
-// kernel has finished and its writes are visible, and only then lets the next
-// kernel's CTAs start.  Every thread of every kernel launched this way calls
-// it before it leaves, so kernels finish in stream order, and before it,
-// a kernel reads only what was written two or more launches earlier and
-// writes nothing.  (In a kernel launched the ordinary way it returns at once.)
+// kernel has finished and its writes are visible.  Every thread of every
+// kernel launched this way calls it before it leaves, so a kernel finishes
+// after all before it, and their writes are visible behind the wait too.
+// Before it a kernel writes nothing and reads only what no launch of the chain
+// writes: links, clover blocks, shifts, hopping parameters.  What an earlier
+// launch of the chain wrote, however far back, is read behind the wait: only
+// there is it known to be visible.  (The one exception is a flag read for a
+// hint, retired() in views.cuh.)  In a kernel launched the ordinary way the
+// wait returns at once.
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ void chain_wait() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -198,7 +202,7 @@ __device__ __forceinline__ void chain_wait() {
 }
 
 // p, as known only after the chain_wait before: no load through it can be
-// moved ahead of the wait
+// moved ahead of the wait (the loads of ld_field could otherwise be)
 template <typename T>
 __device__ __forceinline__ T* after_wait(T* p) {
   asm volatile("" : "+l"(p)::"memory");
@@ -209,10 +213,10 @@ __device__ __forceinline__ T* after_wait(T* p) {
 // field views
 // ---------------------------------------------------------------------------
 // spinor loads: ld.global, not the read-only path (ld.global.nc), since a
-// chained kernel starts before the field it gathers from is written; the
-// compiler may reorder them like read-only loads, and takes those of a field
-// that the launch before writes through a pointer from after_wait.  (As plain
-// C++ loads k_pass2<int16> at 32^3x64 took 111 instead of 104 us.)
+// chained kernel starts before the fields it reads are written; the compiler
+// may reorder them like read-only loads, so a chained kernel takes its fields
+// through pointers from after_wait.  (As plain C++ loads k_pass2<int16> at
+// 32^3x64 took 111 instead of 104 us.)
 __device__ __forceinline__ double2 ld_field(const double2* p) {
   double2 r;
   asm("ld.global.v2.f64 {%0, %1}, [%2];" : "=d"(r.x), "=d"(r.y) : "l"(p));
@@ -1084,32 +1088,31 @@ __device__ __forceinline__ void wilson_hop(const Geom& g, int e, int i, const Si
 // 24 link words (8 hops x 3) are requested before any neighbour spinor, so
 // they stream from HBM while the gathers, which mostly hit L2, proceed hop by
 // hop.  Same products in the same order as wilson_hop, so the result is
-// bit-identical; it needs about 40 more registers.
-// WAIT: the gathered field is written by the launch before (chain_wait).
-template <bool DAG, bool WAIT = true>
-__device__ __forceinline__ void wilson_hop_lf(const Geom& g, int e, int i, const Site& st,
-                                              const SpinorView<Prec::F16>& in0, const GaugeView<Prec::F16>& U,
-                                              Spinor<float>& b, float hscale = 1.f) {
+// bit-identical; it needs about 40 more registers.  load_hop_links may run
+// before chain_wait (no chained launch writes links), wilson_hop_lf not.
+struct HopLinks {
+  uint2 w[4][2][3];
+  int j[4][2];  // neighbours
+};
+__device__ __forceinline__ void load_hop_links(const Geom& g, int e, int i, const Site& st,
+                                               const GaugeView<Prec::F16>& U, HopLinks& l) {
   const int o = 1 - e;
   const uint2* ub = reinterpret_cast<const uint2*>(U.v);
   const int S = U.stride;
-  uint2 W[4][2][3];
-  int J[4][2];
 #pragma unroll
   for (int mu = 3; mu >= 0; mu--) {
-    J[mu][0] = neighbour(g, st, i, mu, true);
-    J[mu][1] = neighbour(g, st, i, mu, false);
+    l.j[mu][0] = neighbour(g, st, i, mu, true);
+    l.j[mu][1] = neighbour(g, st, i, mu, false);
 #pragma unroll
     for (int w = 0; w < 3; w++) {
-      W[mu][0][w] = ld_once(ub + (size_t)((mu * 2 + e) * 3 + w) * S + i);
-      W[mu][1][w] = ld_once(ub + (size_t)((mu * 2 + o) * 3 + w) * S + J[mu][1]);
+      l.w[mu][0][w] = ld_once(ub + (size_t)((mu * 2 + e) * 3 + w) * S + i);
+      l.w[mu][1][w] = ld_once(ub + (size_t)((mu * 2 + o) * 3 + w) * S + l.j[mu][1]);
     }
   }
-  SpinorView<Prec::F16> in = in0;
-  if constexpr (WAIT) {
-    chain_wait();  // the links do not depend on the launch before
-    in = after_wait(in0);
-  }
+}
+template <bool DAG>
+__device__ __forceinline__ void wilson_hop_lf(const Geom& g, const Site& st, const HopLinks& l,
+                                              const SpinorView<Prec::F16>& in, Spinor<float>& b, float hscale = 1.f) {
 #pragma unroll
   for (int mu = 3; mu >= 0; mu--) {
 #pragma unroll
@@ -1118,14 +1121,14 @@ __device__ __forceinline__ void wilson_hop_lf(const Geom& g, int e, int i, const
       cx<float> h[2][3], f[2][3];
       float sc, lsc;
       if (mu == 3) {
-        in.load_pair_raw(J[mu][fb], fwd ? (DAG ? 0 : 2) : (DAG ? 2 : 0), h, sc);
+        in.load_pair_raw(l.j[mu][fb], fwd ? (DAG ? 0 : 2) : (DAG ? 2 : 0), h, sc);
       } else {
         float2 F[4][3];
-        in.load_biased(J[mu][fb], F, sc);
+        in.load_biased(l.j[mu][fb], F, sc);
         project_biased<DAG>(F, mu, fwd, h);
       }
       Link<float> u;
-      links16_decode(W[mu][fb][0], W[mu][fb][1], W[mu][fb][2], u, lsc);
+      links16_decode(l.w[mu][fb][0], l.w[mu][fb][1], l.w[mu][fb][2], u, lsc);
       const float k = (float)hop_sign(g, st, mu, fwd) * sc * lsc * hscale;
       if (fwd) {
         mul_u(u, h, f);

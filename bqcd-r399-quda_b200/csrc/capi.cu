@@ -252,8 +252,8 @@ int cg_core(bqcdg_ctx* c, double2* x, double2* b, const OpParams& op, Prec slopp
       // the fused update leaves the stepped scalars in the other of two slots;
       // a batch is even, so it ends in slot 0
       CgScalars *cg = c->dcg + (fused ? k & 1 : 0), *next = c->dcg + (~k & 1);
-      // what pass 1 may read before its wait: the slot that the launch before
-      // it does not write (it then runs once in vain when the solve stops)
+      // pass 1 asks the slot that the launch before it does not write (when the
+      // solve stops it then runs once in vain, into scratch)
       const CgScalars* prev = fused && k > 0 ? next : cg;
       if (timed) kt.begin();
       launch_mtil_pass1(sloppy, gs, false, t, p, gauge_of(c, sloppy), ainv_of(c, sloppy), op, prev, c->stream, 1,

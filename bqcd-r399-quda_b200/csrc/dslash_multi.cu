@@ -199,13 +199,10 @@ __global__ void __launch_bounds__(kBlock, OccN<NB>::min_blocks)
   const GTile tl = gtile(ng, fin.partial ? 1 : 0);
   const int rhs0 = tl.grp * NB;
   bool act[NB];
-  if (!group_live<NB>(cg, rhs0, nr, act)) {
-    chain_wait();
-    return;
-  }
+  chain_wait();
+  if (!group_live<NB>(cg, rhs0, nr, act)) return;
   if (tl.sb < 0) {
     // alpha of the k_pass2_n before (defer_alpha), as in k_pass1
-    chain_wait();
     double tot[NB];
     final_sum<NB>(after_wait(fin.partial) + (size_t)rhs0 * kRedVals * fin.stride, kRedVals * fin.stride, tl.nsb, tot);
     if (threadIdx.x == 0) {
@@ -218,21 +215,15 @@ __global__ void __launch_bounds__(kBlock, OccN<NB>::min_blocks)
     return;
   }
   const int i = tl.i;
-  if (i >= g.volh) {
-    chain_wait();
-    return;
-  }
+  if (i >= g.volh) return;
   SpinorView<P> in[NB];
 #pragma unroll
-  for (int r = 0; r < NB; r++) in[r] = sview<P>(rhs_of(inp, rhs0 + r), g.stride);
+  for (int r = 0; r < NB; r++) in[r] = after_wait(sview<P>(rhs_of(inp, rhs0 + r), g.stride));
   auto U = gview<P>(gauge, g);
   const Site st = site_coords(g, i, 1);
   Spinor<R> b[NB];
 #pragma unroll
   for (int r = 0; r < NB; r++) zero(b[r]);
-  chain_wait();
-#pragma unroll
-  for (int r = 0; r < NB; r++) in[r] = after_wait(in[r]);
   wilson_hop_n<P, DAG, NB>(g, 1, i, st, in, act, U, b, (R)1);
   R osc = 1;  // a common factor of the outputs, folded into their storage scale
   if (has_clover) {
@@ -311,11 +302,7 @@ __device__ __forceinline__ void pass2_core_n(const Geom& g, int i, const SpinorV
     }
   }
   const Site st = site_coords(g, i, 0);
-  chain_wait();  // t is written by the launch before, x and the clover blocks earlier
-  SpinorView<P> tw[NB];
-#pragma unroll
-  for (int r = 0; r < NB; r++) tw[r] = after_wait(t[r]);
-  wilson_hop_n<P, DAG, NB>(g, 0, i, st, tw, act, U, out, (R)bcoef);
+  wilson_hop_n<P, DAG, NB>(g, 0, i, st, t, act, U, out, (R)bcoef);
 }
 
 // the shifts of the group's right-hand sides
@@ -337,10 +324,8 @@ __global__ void __launch_bounds__(kBlock, OccN<NB>::min_blocks)
   const GTile tl = gtile(ng);
   const int rhs0 = tl.grp * NB;
   bool act[NB];
-  if (!group_live<NB>(cg, rhs0, nr, act)) {
-    chain_wait();
-    return;
-  }
+  chain_wait();
+  if (!group_live<NB>(cg, rhs0, nr, act)) return;
   double rh[NB];
   group_rho<NB>(rho, rho_rhs, rhs0, act, rh);
   const int i = tl.i;
@@ -351,8 +336,8 @@ __global__ void __launch_bounds__(kBlock, OccN<NB>::min_blocks)
     SpinorView<P> t[NB], x[NB];
 #pragma unroll
     for (int r = 0; r < NB; r++) {
-      t[r] = sview<P>(rhs_of(tp, rhs0 + r), g.stride);
-      x[r] = sview<P>(rhs_of(xp, rhs0 + r), g.stride);
+      t[r] = after_wait(sview<P>(rhs_of(tp, rhs0 + r), g.stride));
+      x[r] = after_wait(sview<P>(rhs_of(xp, rhs0 + r), g.stride));
     }
     Spinor<R> o[NB];
     pass2_core_n<P, false, NB>(g, i, t, x, act, gview<P>(gauge, g), aee, has_clover, bcoef, rh, o);
@@ -365,8 +350,6 @@ __global__ void __launch_bounds__(kBlock, OccN<NB>::min_blocks)
 #pragma unroll
         for (int c = 0; c < 3; c++) acc[r] += (double)norm2(o[r].c[s][c]);
     }
-  } else {
-    chain_wait();
   }
   // value r of the group goes to the partial slot of RHS rhs0 + r
   double* part = red.partial + (size_t)rhs0 * kRedVals * red.maxblocks;
@@ -411,10 +394,8 @@ __global__ void __launch_bounds__(kBlock, OccN<NB>::min_blocks)
   const GTile tl = gtile(ng);
   const int rhs0 = tl.grp * NB;
   bool act[NB];
-  if (!group_live<NB>(cgs, rhs0, nr, act)) {
-    chain_wait();
-    return;
-  }
+  chain_wait();
+  if (!group_live<NB>(cgs, rhs0, nr, act)) return;
   double rh[NB];
   group_rho<NB>(rho, rho_rhs, rhs0, act, rh);
   const int i = tl.i;
@@ -425,15 +406,15 @@ __global__ void __launch_bounds__(kBlock, OccN<NB>::min_blocks)
     SpinorView<P> t[NB], q[NB];
 #pragma unroll
     for (int r = 0; r < NB; r++) {
-      t[r] = sview<P>(rhs_of(tp, rhs0 + r), g.stride);
-      q[r] = sview<P>(rhs_of(qp, rhs0 + r), g.stride);
+      t[r] = after_wait(sview<P>(rhs_of(tp, rhs0 + r), g.stride));
+      q[r] = after_wait(sview<P>(rhs_of(qp, rhs0 + r), g.stride));
     }
     Spinor<R> ap[NB];
     pass2_core_n<P, true, NB>(g, i, t, q, act, gview<P>(gauge, g), aee, has_clover, bcoef, rh, ap);
 #pragma unroll
     for (int r = 0; r < NB; r++) {
       if (!act[r]) continue;
-      const auto rv = sview<Prec::F32>(rhs_of(rp, rhs0 + r), g.stride);
+      const auto rv = after_wait(sview<Prec::F32>(rhs_of(rp, rhs0 + r), g.stride));
       const float a = (float)cgs[rhs0 + r].alpha;
       Spinor<float> rl;
       rv.load(i, rl);
@@ -446,8 +427,6 @@ __global__ void __launch_bounds__(kBlock, OccN<NB>::min_blocks)
         }
       rv.store(i, rl);
     }
-  } else {
-    chain_wait();
   }
   double* part = red.partial + (size_t)rhs0 * kRedVals * red.maxblocks;
   block_reduce_store<NB>(acc, part, kRedVals * red.maxblocks, tl.sb);

@@ -89,20 +89,15 @@ __global__ void __launch_bounds__(128, 3)
   const int chi = warp >> 1, s = warp & 1;
   const int extra = fin.partial ? 1 : 0;
   const int rhs = blockIdx.x % nr, sb = (int)(blockIdx.x / nr) - extra, nsb = gridDim.x / nr - extra;
-  if (cgs && cgs[rhs].done) {  // retired right-hand side
-    chain_wait();
-    return;
-  }
   if (sb < 0) {
     // alpha of the second pass before (k_pass1's extra CTA)
     chain_wait();
     double tot[1];
     final_sum<1>(after_wait(fin.partial) + (size_t)rhs * kRedVals * fin.stride, fin.stride, nsb, tot);
-    if (threadIdx.x == 0) {
-      cg_set_alpha(fin.cg + rhs, tot[0]);
-    }
+    if (threadIdx.x == 0 && !fin.cg[rhs].done) cg_set_alpha(fin.cg + rhs, tot[0]);
     return;
   }
+  if (retired(cgs ? cgs + rhs : nullptr)) return;
   // threads beyond the last site work on it too, and store nothing
   const int i0 = sb * kSplitSites + lane;
   const bool live = i0 < g.volh;
@@ -111,35 +106,9 @@ __global__ void __launch_bounds__(128, 3)
   const auto U = gview<P>(gauge, g);
   const Site st = site_coords(g, i, e);
 
-  // the site-local terms of the second passes: rows of A_ee x and of rho x
-  cx<R> z[3];
-#pragma unroll
-  for (int c = 0; c < 3; c++) z[c] = mkc<R>(0, 0);
-  if constexpr (W != Pass::First) {
-    const auto xin = sview<P>(rhs_of(xp, rhs), g.stride);
-    Spinor<R> x;
-    xin.load(i, x);
-    cx<R> xc[6];
-#pragma unroll
-    for (int k = 0; k < 6; k++)
-      xc[k] = chi == 0 ? x.c[k / 3][k % 3] + x.c[k / 3 + 2][k % 3] : x.c[k / 3][k % 3] - x.c[k / 3 + 2][k % 3];
-    // x itself is half the sum (difference) of its chiral parts
-    const R own = 0.5 * (rho + (has_clover ? 0.0 : 1.0));
-    if (has_clover) {
-      cx<R> a[18];
-      load_rows(cview<P>(ap, g.stride), i, chi, s, a);
-      rows_mv(s, a, xc, z);
-    }
-#pragma unroll
-    for (int c = 0; c < 3; c++) {
-      const cx<R> xo = s == 0 ? xc[c] : xc[3 + c];
-      z[c] = z[c] + own * xo;
-      if (!has_clover && hval != 0.0) z[c] = z[c] + (chi == 0 ? 0.5 : -0.5) * hval * itimes(xo);
-    }
-  }
   chain_wait();
+  const bool stopped = cgs && cgs[rhs].done;
   const auto t = after_wait(sview<P>(rhs_of(tp, rhs), g.stride));
-
   Spinor<R> b;
   zero(b);
   const R hs = W == Pass::First ? 1.0 : bcoef;
@@ -153,8 +122,29 @@ __global__ void __launch_bounds__(128, 3)
     part[warp][k][lane] = make_double2(u.x + d.x, u.y + d.y);
     part[warp][6 + k][lane] = make_double2(u.x - d.x, u.y - d.y);
   }
-  cx<R> a[18];
-  if (W == Pass::First && has_clover) load_rows(cview<P>(ap, g.stride), i, chi, s, a);
+  cx<R> a[18], z[3];  // rows of A_ee or A_oo^-1
+  if (has_clover) load_rows(cview<P>(ap, g.stride), i, chi, s, a);
+#pragma unroll
+  for (int c = 0; c < 3; c++) z[c] = mkc<R>(0, 0);
+  if constexpr (W != Pass::First) {
+    // the site-local terms: rows of A_ee x and of rho x
+    Spinor<R> x;
+    after_wait(sview<P>(rhs_of(xp, rhs), g.stride)).load(i, x);
+    cx<R> xc[6];
+#pragma unroll
+    for (int k = 0; k < 6; k++)
+      xc[k] = chi == 0 ? x.c[k / 3][k % 3] + x.c[k / 3 + 2][k % 3] : x.c[k / 3][k % 3] - x.c[k / 3 + 2][k % 3];
+    // x itself is half the sum (difference) of its chiral parts
+    const R own = 0.5 * (rho + (has_clover ? 0.0 : 1.0));
+    if (has_clover) rows_mv(s, a, xc, z);
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+      const cx<R> xo = s == 0 ? xc[c] : xc[3 + c];
+      z[c] = z[c] + own * xo;
+      if (!has_clover && hval != 0.0) z[c] = z[c] + (chi == 0 ? 0.5 : -0.5) * hval * itimes(xo);
+    }
+  }
+  if (stopped) return;
   __syncthreads();
   if (W == Pass::First && has_clover) {
     // every row needs the whole chiral vector
@@ -198,7 +188,7 @@ __global__ void __launch_bounds__(128, 3)
   }
   const int sp = s + 2 * chi;
   double acc[1] = {0.0};
-  const auto out = sview<P>(rhs_of(outp, rhs), g.stride);
+  const auto out = after_wait(sview<P>(rhs_of(outp, rhs), g.stride));
   if (W == Pass::Cg) {
     const R al = cgs[rhs].alpha;  // set by the launch before
 #pragma unroll

@@ -35,11 +35,8 @@ struct RedScratch {
   int maxblocks = 0;
 };
 
-// scalars of a CG kept in device memory (no host round trip per iteration).
-// alpha and live, which the second half of an iteration reads, have a cache
-// line of their own: the CG step writes the first line while k_cg_pupdate,
-// launched behind it (launch_chain), already reads the second.
-struct alignas(256) CgScalars {
+// scalars of a CG kept in device memory (no host round trip per iteration)
+struct CgScalars {
   double rtr;       // |r|^2 after the latest update
   double rtr_old;   // |r|^2 of the previous iteration
   double beta;
@@ -51,7 +48,7 @@ struct alignas(256) CgScalars {
   int done;         // 0 running, 1 converged, 2 reliable update requested, 3 maxiter, 4 NaN
   int last_ru;      // iteration of the last reliable update
   int ru_every;     // also update after this many iterations without one (0: never)
-  alignas(128) double paap;  // p.(A p) = |M p|^2
+  double paap;      // p.(A p) = |M p|^2
   double alpha;
   int live;         // the iteration that alpha belongs to (iter + 1 when it was set)
 };
@@ -66,13 +63,14 @@ struct OpParams {
 // A launch that may start while the kernel before it in the stream drains
 // (programmatic stream serialization), when chain is set.  Only for kernels
 // whose threads all call chain_wait (bqcdg_internal.cuh, which has the rules),
-// and only where the launch before does not write the links, the clover
+// and only where no launch chained before it writes the links, the clover
 // fields or whatever else the kernel reads before chain_wait.  Without it
-// about 2.2 us pass between two launches; with it the next kernel's index
-// arithmetic, links, clover blocks and local spinor are on their way by then.
-// Mixed solves: 18.7 -> 12.9 ms at 16^3x32, 6.6 -> 4.6 ms at 10x6x14x18; FP64
-// CG: 9.0 -> 6.7 ms at 8^4, 173.4 -> 169.9 ms at 24^3x48; at 32^3x64, where a
-// launch takes 100 us, no change.
+// about 2.2 us pass between two launches; with it the next kernel's CTAs are
+// resident by then, with their index arithmetic done and, in the int16 passes,
+// their links on their way.  Mixed solves: 19.1 -> 13.5 ms at 16^3x32, 10.6 ->
+// 7.1 ms at 10x6x14x18, 248 -> 244 ms at 32^3x64; FP64 CG: 5.7 -> 4.0 ms at
+// 8^4, 175 -> 172 ms at 24^3x48; FP32: Wilson at 12x20x28x36 8.4 -> 6.7 ms, 12
+// systems at 12^3x24 48.3 -> 43.2 ms.
 template <typename... KP, typename... A>
 inline void launch_chain(bool chain, void (*k)(KP...), dim3 grid, int block, cudaStream_t s, A... a) {
   cudaLaunchAttribute at{};
