@@ -237,7 +237,7 @@ int cg_core(bqcdg_ctx* c, double2* x, double2* b, const OpParams& op, Prec slopp
   int batch = 4;
   const Geom& gs = geom_of(c, sloppy);  // stencil geometry (12-real FP64 links when SU(3))
   const int nsb = site_blocks(sloppy, gs);  // block partials of a pass
-  const bool fused = nsb <= kFusedStep;
+  const bool fused = fused_step(sloppy, nsb);
   while (!h.done) {
     nl += (fused ? 5 : 6) * batch;
     const int iter0 = h.iter;

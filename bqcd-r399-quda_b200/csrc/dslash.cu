@@ -556,9 +556,9 @@ void launch_cg_pupdate(Prec p, const Geom& g, SpinorPtr pvec, SpinorPtr r, CgSca
 // k_cg_step and k_cg_pupdate in one launch, for one right-hand side: every CTA
 // sums the |r|^2 partials of the launch before and takes the scalar step for
 // itself, CTA 0 stores it.  It goes to `next`, which the following iteration
-// reads, since other CTAs still read `cur`.  At most kFusedStep CTAs, which two
-// per SM hold, so nothing has to spill (for 3 to 5 per SM 32 to 48 bytes: FP64
-// CG at 8^4 4.34 instead of 4.13 ms).
+// reads, since other CTAs still read `cur`.  At most 256 CTAs (fused_step),
+// which two per SM hold, so nothing has to spill (for 3 to 5 per SM 32 to 48
+// bytes: FP64 CG at 8^4 4.34 instead of 4.13 ms).
 template <Prec P, Prec RP>
 __global__ void __launch_bounds__(kBlock, 2) k_cg_update(Geom g, SpinorPtr pp, SpinorPtr rp, SpinorPtr xp,
                                                       const CgScalars* cur, CgScalars* next, RedScratch red, int nsb) {

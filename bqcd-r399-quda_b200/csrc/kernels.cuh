@@ -175,12 +175,14 @@ void launch_split_pass4(const Geom& g, SpinorPtr t, SpinorPtr q, const void* gau
 void launch_cg_pupdate(Prec p, const Geom& g, SpinorPtr pvec, SpinorPtr r, CgScalars* cg, cudaStream_t s,
                        int nr, SpinorPtr x, const CgExpect& expect, bool chain = false);
 
-// both, for one right-hand side and up to kFusedStep block partials: every CTA
-// sums them itself.  The stepped scalars go to `next`; when the iteration did
-// not run they are those of `cur`.  At 60 partials a mixed solve (10x6x14x18)
-// takes 4.4 instead of 4.7 ms and FP64 CG at 8^4 3.8 instead of 4.0 ms; at 512
-// and 945 the sums cost what the launch saves (12.9, 6.9 ms -> 13.0, 7.0 ms).
-constexpr int kFusedStep = 2 * kBlock;
+// both, for one right-hand side: every CTA sums the partials itself.  The
+// stepped scalars go to `next`; when the iteration did not run they are those
+// of `cur`.  One launch less, at one more reading of all partials per CTA.  Per
+// iteration, apart and together: FP64 24.6 and 21.4 us at 64 partials (8^4),
+// 32.2 and 30.5 at 256, FP32 57 and 54 at 256, int16 37.9 and 34.5 at 60
+// (10x6x14x18), 40.3 and 37.1 at 215, 43.4 and 43.4 at 224, but 41.4 and 44.3
+// at 236 and 43.5 and 48.8 at 256; from 384 on FP32 loses as well.
+inline bool fused_step(Prec p, int nsb) { return nsb <= (p == Prec::F16 ? 216 : 256); }
 void launch_cg_update(Prec p, const Geom& g, SpinorPtr pvec, SpinorPtr r, SpinorPtr x, const CgScalars* cur,
                       CgScalars* next, RedScratch red, int nsb, cudaStream_t s);
 
