@@ -17,15 +17,22 @@ namespace bqcdg {
 
 constexpr int kSplitSites = 32;
 
-// FP64 fields below one wave of the one-thread passes (222 to 248 registers:
-// 2 CTAs of 128 sites on each of 148 SMs).  Above it the shared-memory
-// exchange costs more than the shorter chain saves: FP64 CG 6.7 -> 4.1 ms at
-// 8^4, 12 systems' updates at 12^3x24 (20736 sites) 46.5 -> 45.3 ms for the
-// solve, no change at 16^3x32 (65536 sites), 169.9 -> 179.3 ms at 24^3x48.
+// FP64 fields that the one-thread passes (222 to 248 registers: 2 CTAs of 128
+// sites per SM) do in one wave, where the CTAs here, 3 per SM, come to at most
+// three per SM for each of theirs: both take a step in time with each CTA more
+// on an SM or wave more.  Per FP64 CG iteration with four threads and with one:
+//     2048 sites of a parity 21.4 and 40 us, 13824 32.6 and 44.1 (one wave here)
+//    17280                   47.3 and 45.1 (two waves, one CTA per SM there)
+//    20736                   49.9 and 54.4, 27648 53.5 and 59.0 (two and two)
+//    30184                   69.8 and 60.5, 36864 76.3 and 66.8 (three waves)
+// and a 24^3x48 solve 179 and 170 ms.
 // Four threads per site did nothing for int16 at 10x6x14x18 and slowed the
 // FP32 and int16 passes of larger lattices, which wait on issue, not latency.
 bool split_sites(Prec p, const Geom& g) {
-  return p == Prec::F64 && !g.clover_t && g.volh <= 148 * 2 * kBlock;
+  constexpr int kSMs = 148;
+  const int one = ((g.volh + kBlock - 1) / kBlock + kSMs - 1) / kSMs;
+  const int four = ((g.volh + kSplitSites - 1) / kSplitSites + kSMs - 1) / kSMs;
+  return p == Prec::F64 && !g.clover_t && one <= 2 && four <= 3 * one;
 }
 int site_blocks(Prec p, const Geom& g) {
   return split_sites(p, g) ? (g.volh + kSplitSites - 1) / kSplitSites : nblocks(g.volh);

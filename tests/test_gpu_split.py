@@ -1,7 +1,8 @@
 """The FP64 passes with four threads per site (dslash_split.cu) against the
 CPU oracle: a single CTA with idle lanes (8 sites), a remainder of 8 sites in
-the last CTA, and a lattice on each side of the size up to which they are
-taken (37888 sites of a parity), with every term of the operators.
+the last CTA, and lattices on each side of every bound of split_sites (14208,
+18944 and 28416 sites of a parity; beyond, the one-thread passes in one wave and
+in two), with every term of the operators.
 Relative norm-wise agreement to 1e-13: some 1,400 FP64 operations per site and
 pass, rounding to 2^-53 each."""
 import numpy as np
@@ -9,7 +10,8 @@ import pytest
 
 pytestmark = pytest.mark.gpu
 
-LATTICES = [(2, 2, 2, 2), (6, 6, 6, 6), (16, 16, 16, 18), (20, 16, 16, 16)]
+LATTICES = [(2, 2, 2, 2), (6, 6, 6, 6), (12, 12, 12, 16), (12, 12, 10, 20), (12, 12, 12, 22), (12, 12, 16, 24),
+            (14, 14, 14, 22), (16, 16, 16, 18), (20, 16, 16, 16)]
 
 
 def rel(a, b):
