@@ -431,9 +431,31 @@ int read_residuals(bqcdg_ctx* c, int nb) {
   return BQCDG_OK;
 }
 
+// the four stencil passes of a batched CG iteration over the batch buffers,
+// nbt right-hand sides per thread (1: one per CTA), each with its own shift and
+// hopping parameter where rho and kappa (device) are given
+void queue_passes(bqcdg_ctx* c, Prec p, const OpParams& op, int nb, int nbt, const double* rho, const double* kappa) {
+  auto& B = c->batch;
+  const Geom& g = c->g;
+  const void* U = gauge_of(c, p);
+  const AlphaFin fin{c->red.partial, c->red.maxblocks, c->dcg};
+  if (nbt > 1) {
+    launch_mtil_pass1_n(p, g, false, B.t, B.p, U, ainv_of(c, p), op, c->dcg, c->stream, nb, nbt, AlphaFin{}, true);
+    launch_mtil_pass2_n(p, g, B.q, B.t, B.p, U, aee_of(c, p), op, c->red, c->dcg, c->stream, nb, rho, nbt, true, true);
+    launch_mtil_pass1_n(p, g, true, B.t, B.q, U, ainv_of(c, p), op, c->dcg, c->stream, nb, nbt, fin, true);
+    launch_cg_pass4_n(p, g, B.t, B.q, U, aee_of(c, p), op, B.rs, c->red, c->dcg, c->stream, nb, rho, nbt, true, true);
+  } else {
+    launch_mtil_pass1(p, g, false, B.t, B.p, U, ainv_of(c, p), op, c->dcg, c->stream, nb, kappa, AlphaFin{}, true);
+    launch_mtil_pass2(p, g, false, B.q, B.t, B.p, U, aee_of(c, p), op, c->red, nullptr, c->dcg, c->stream, nb, rho,
+                      kappa, true, true);
+    launch_mtil_pass1(p, g, true, B.t, B.q, U, ainv_of(c, p), op, c->dcg, c->stream, nb, kappa, fin, true);
+    launch_cg_pass4(p, g, B.t, B.q, U, aee_of(c, p), op, B.rs, c->red, c->dcg, c->stream, nb, rho, kappa, true, true);
+  }
+}
+
 int tune_nbt(bqcdg_ctx* c, Prec p, const OpParams& op, int nb, int* nbt, float* ms = nullptr);
 
-// Batched mixed-precision CG over nb right-hand sides: the five kernels of a
+// Batched mixed-precision CG over nb right-hand sides: the six kernels of a
 // sloppy iteration each serve all nb (CTAs rhs-fastest), every right-hand
 // side has its own scalars, stops and FP64 reliable updates, and a converged
 // or paused one costs its CTAs an early return only.  nbt: right-hand sides
@@ -509,27 +531,8 @@ int cg_batch(bqcdg_ctx* c, double2** x, double2** b, int nb, const OpParams& op,
     for (int k = 0; k < nb; k++) expect.n[k] = c->hcg[k].iter;
     for (int it = 0; it < batch; it++) {
       for (int k = 0; k < nb; k++) expect.n[k]++;
-      if (nbt > 1) {
-        launch_mtil_pass1_n(sloppy, g, false, B.t, B.p, gauge_of(c, sloppy), ainv_of(c, sloppy), op, c->dcg,
-                            c->stream, nb, nbt, AlphaFin{}, true);
-        launch_mtil_pass2_n(sloppy, g, B.q, B.t, B.p, gauge_of(c, sloppy), aee_of(c, sloppy), op, c->red, c->dcg,
-                            c->stream, nb, drho, nbt, true, true);
-        launch_mtil_pass1_n(sloppy, g, true, B.t, B.q, gauge_of(c, sloppy), ainv_of(c, sloppy), op, c->dcg,
-                            c->stream, nb, nbt, AlphaFin{c->red.partial, c->red.maxblocks, c->dcg}, true);
-        launch_cg_pass4_n(sloppy, g, B.t, B.q, gauge_of(c, sloppy), aee_of(c, sloppy), op, B.rs, c->red, c->dcg,
-                          c->stream, nb, drho, nbt, true, true);
-        launch_cg_step(c->red, c->dcg, nb, nblocks(g.volh), c->stream);
-      } else {
-        launch_mtil_pass1(sloppy, g, false, B.t, B.p, gauge_of(c, sloppy), ainv_of(c, sloppy), op, c->dcg,
-                          c->stream, nb, dkap, AlphaFin{}, true);
-        launch_mtil_pass2(sloppy, g, false, B.q, B.t, B.p, gauge_of(c, sloppy), aee_of(c, sloppy), op, c->red,
-                          nullptr, c->dcg, c->stream, nb, drho, dkap, true, true);
-        launch_mtil_pass1(sloppy, g, true, B.t, B.q, gauge_of(c, sloppy), ainv_of(c, sloppy), op, c->dcg,
-                          c->stream, nb, dkap, AlphaFin{c->red.partial, c->red.maxblocks, c->dcg}, true);
-        launch_cg_pass4(sloppy, g, B.t, B.q, gauge_of(c, sloppy), aee_of(c, sloppy), op, B.rs, c->red, c->dcg,
-                        c->stream, nb, drho, dkap, true, true);
-        launch_cg_step(c->red, c->dcg, nb, dkap ? nblocks(g.volh) : site_blocks(sloppy, g), c->stream);
-      }
+      queue_passes(c, sloppy, op, nb, nbt, drho, dkap);
+      launch_cg_step(c->red, c->dcg, nb, nblocks(g.volh), c->stream);
       launch_cg_pupdate(sloppy, g, B.p, B.rs, c->dcg, c->stream, nb, B.xs, expect, true);
     }
     launches += 6 * batch;
@@ -637,28 +640,13 @@ int time_pass1(bqcdg_ctx* c, Prec p, const OpParams& op, int nb, int nbt, int re
   return BQCDG_OK;
 }
 
-// device time of one batched M~^+M~ over the batch buffers (the four stencil
-// passes of a CG iteration, the second halves with their reductions but no
-// CG scalars), nbt right-hand sides per thread.  The buffers hold no solve
-// while the tuner runs.
-int time_mdagm_batch(bqcdg_ctx* c, Prec p, const OpParams& op, int nb, int nbt, int reps, float* ms) {
-  auto& B = c->batch;
-  const void* U = gauge_of(c, p);
-  auto launch = [&]() {
-    if (nbt > 1) {
-      launch_mtil_pass1_n(p, c->g, false, B.t, B.p, U, ainv_of(c, p), op, nullptr, c->stream, nb, nbt);
-      launch_mtil_pass2_n(p, c->g, B.q, B.t, B.p, U, aee_of(c, p), op, c->red, nullptr, c->stream, nb, nullptr, nbt,
-                          true);
-      launch_mtil_pass1_n(p, c->g, true, B.t, B.q, U, ainv_of(c, p), op, nullptr, c->stream, nb, nbt);
-      launch_mtil_pass2_n(p, c->g, B.p, B.t, B.q, U, aee_of(c, p), op, c->red, nullptr, c->stream, nb, nullptr, nbt,
-                          true);
-    } else {
-      launch_mtil_pass1(p, c->g, false, B.t, B.p, U, ainv_of(c, p), op, nullptr, c->stream, nb);
-      launch_mtil_pass2(p, c->g, false, B.q, B.t, B.p, U, aee_of(c, p), op, c->red, nullptr, nullptr, c->stream, nb);
-      launch_mtil_pass1(p, c->g, true, B.t, B.q, U, ainv_of(c, p), op, nullptr, c->stream, nb);
-      launch_mtil_pass2(p, c->g, true, B.p, B.t, B.q, U, aee_of(c, p), op, c->red, nullptr, nullptr, c->stream, nb);
-    }
-  };
+// device time of the four stencil passes of one batched CG iteration, as the
+// solver queues them, nbt right-hand sides per thread.  The batch buffers hold
+// no solve while the tuner runs; with zero scalars no right-hand side stops
+// and alpha changes no launch's work.
+int time_passes(bqcdg_ctx* c, Prec p, const OpParams& op, int nb, int nbt, int reps, float* ms) {
+  CK(cudaMemsetAsync(c->dcg, 0, sizeof(CgScalars) * nb, c->stream));
+  auto launch = [&]() { queue_passes(c, p, op, nb, nbt, nullptr, nullptr); };
   launch();
   CK(cudaEventRecord(c->ev0, c->stream));
   for (int r = 0; r < reps; r++) launch();
@@ -672,8 +660,8 @@ int time_mdagm_batch(bqcdg_ctx* c, Prec p, const OpParams& op, int nb, int nbt, 
 }
 
 // right-hand sides per stencil thread for launches of nb at precision p:
-// the fastest batched M~^+M~ of 1, 2 and 4 (timed once, then cached).  The
-// register-blocked passes need h = 0.  ms: the chosen time, when timed.
+// the fastest passes of an iteration of 1, 2 and 4 (timed once, then cached).
+// The register-blocked passes need h = 0.  ms: the chosen time, when timed.
 int tune_nbt(bqcdg_ctx* c, Prec p, const OpParams& op, int nb, int* nbt, float* ms) {
   int& cached = c->tuned_nbt[(int)p][nb];
   if (cached && !ms) {
@@ -685,7 +673,7 @@ int tune_nbt(bqcdg_ctx* c, Prec p, const OpParams& op, int nb, int* nbt, float* 
   for (int k : {1, 2, 4}) {
     if (k > 1 && (k > nb || op.h != 0.0 || p == Prec::F64 || c->g.clover_t)) break;
     float t;
-    int st = time_mdagm_batch(c, p, op, nb, k, 2, &t);
+    int st = time_passes(c, p, op, nb, k, 2, &t);
     if (st) return st;
     if (k == 1 || t < 0.98f * best) {
       best = t;
@@ -698,8 +686,8 @@ int tune_nbt(bqcdg_ctx* c, Prec p, const OpParams& op, int nb, int* nbt, float* 
   return BQCDG_OK;
 }
 
-// RHS per launch for a batch: the per-RHS time of a batched M~^+M~ (at its
-// best RHS per thread), timed for 1, 4, 8 and 16 right-hand sides on the
+// RHS per launch for a batch: the per-RHS time of an iteration's passes (at
+// their best RHS per thread), timed for 1, 4, 8 and 16 right-hand sides on the
 // resident fields
 int tune_block(bqcdg_ctx* c, Prec p, const OpParams& op, int nmax, int* best) {
   const int cand[4] = {1, 4, 8, 16};
