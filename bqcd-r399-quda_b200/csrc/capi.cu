@@ -96,17 +96,18 @@ int check_op(bqcdg_ctx* c, const bqcdg_params* p) {
 // out_e = M~ in_e  (dag: M~^+), with rho for W; t_o scratch (odd)
 // (chain: the launch before is a pass of the same operator)
 void apply_mtil(bqcdg_ctx* c, Prec p, bool dag, SpinorPtr out, SpinorPtr in, SpinorPtr t, const OpParams& op,
-                double* norm_out, CgScalars* cg, bool chain) {
+                bool chain) {
   const Geom& g = geom_of(c, p);
-  launch_mtil_pass1(p, g, dag, t, in, gauge_of(c, p), ainv_of(c, p), op, cg, c->stream, 1, nullptr, AlphaFin{}, chain);
-  launch_mtil_pass2(p, g, dag, out, t, in, gauge_of(c, p), aee_of(c, p), op, c->red, norm_out, cg, c->stream, 1,
-                    nullptr, nullptr, false, true);
+  launch_mtil_pass1(p, g, dag, t, in, gauge_of(c, p), ainv_of(c, p), op, nullptr, c->stream, 1, nullptr, AlphaFin{},
+                    chain);
+  launch_mtil_pass2(p, g, dag, out, t, in, gauge_of(c, p), aee_of(c, p), op, c->red, nullptr, c->stream, 1, nullptr,
+                    nullptr, true);
 }
 
 // out = (W^+ W) in in precision p; scratch t (odd), q (even)
 void apply_mdagm(bqcdg_ctx* c, Prec p, SpinorPtr out, SpinorPtr in, SpinorPtr t, SpinorPtr q, const OpParams& op) {
-  apply_mtil(c, p, false, q, in, t, op, nullptr, nullptr);
-  apply_mtil(c, p, true, out, q, t, op, nullptr, nullptr, true);
+  apply_mtil(c, p, false, q, in, t, op);
+  apply_mtil(c, p, true, out, q, t, op, true);
 }
 
 int read_cg(bqcdg_ctx* c) {
@@ -242,7 +243,7 @@ int cg_core(bqcdg_ctx* c, double2* x, double2* b, const OpParams& op, Prec slopp
     nl += (fused ? 5 : 6) * batch;
     const int iter0 = h.iter;
     for (int k = 0; k < batch; k++) {
-      // pass 1, pass 2 (+|M~p|^2 partials), pass 3 (+ their sum -> alpha), pass 4 (+x,r update, |r|^2
+      // pass 1, pass 2 (+|M~p|^2 partials), pass 3 (+ their sum -> alpha), pass 4 (+r update, |r|^2
       // partials), the CG step, p and x update.  With time_kernels, passes 1 and 3 of the second iteration of
       // each batch are bracketed by events: a sample of every batch in the steady state (the first
       // iteration follows the host's read of the scalars, or a reliable update whose FP64 fields have
@@ -259,14 +260,13 @@ int cg_core(bqcdg_ctx* c, double2* x, double2* b, const OpParams& op, Prec slopp
       launch_mtil_pass1(sloppy, gs, false, t, p, gauge_of(c, sloppy), ainv_of(c, sloppy), op, prev, c->stream, 1,
                         nullptr, AlphaFin{}, true);
       if (timed) kt.end();
-      launch_mtil_pass2(sloppy, gs, false, q, t, p, gauge_of(c, sloppy), aee_of(c, sloppy), op, c->red, nullptr,
-                        cg, c->stream, 1, nullptr, nullptr, true, true);
+      launch_mtil_pass2(sloppy, gs, false, q, t, p, gauge_of(c, sloppy), aee_of(c, sloppy), op, c->red, cg,
+                        c->stream, 1, nullptr, nullptr, true);
       if (timed) kt.begin();
       launch_mtil_pass1(sloppy, gs, true, t, q, gauge_of(c, sloppy), ainv_of(c, sloppy), op, cg, c->stream, 1,
                         nullptr, AlphaFin{c->red.partial, c->red.maxblocks, cg}, true);
       if (timed) kt.end();
-      launch_cg_pass4(sloppy, gs, t, q, gauge_of(c, sloppy), aee_of(c, sloppy), op, rs, c->red, cg, c->stream, 1,
-                      nullptr, nullptr, true, true);
+      launch_cg_pass4(sloppy, gs, t, q, gauge_of(c, sloppy), aee_of(c, sloppy), op, rs, c->red, cg, c->stream);
       if (fused) {
         launch_cg_update(sloppy, g, p, rs, xs, cg, next, c->red, nsb, c->stream);
       } else {
@@ -441,15 +441,15 @@ void queue_passes(bqcdg_ctx* c, Prec p, const OpParams& op, int nb, int nbt, con
   const AlphaFin fin{c->red.partial, c->red.maxblocks, c->dcg};
   if (nbt > 1) {
     launch_mtil_pass1_n(p, g, false, B.t, B.p, U, ainv_of(c, p), op, c->dcg, c->stream, nb, nbt, AlphaFin{}, true);
-    launch_mtil_pass2_n(p, g, B.q, B.t, B.p, U, aee_of(c, p), op, c->red, c->dcg, c->stream, nb, rho, nbt, true, true);
+    launch_mtil_pass2_n(p, g, B.q, B.t, B.p, U, aee_of(c, p), op, c->red, c->dcg, c->stream, nb, rho, nbt);
     launch_mtil_pass1_n(p, g, true, B.t, B.q, U, ainv_of(c, p), op, c->dcg, c->stream, nb, nbt, fin, true);
-    launch_cg_pass4_n(p, g, B.t, B.q, U, aee_of(c, p), op, B.rs, c->red, c->dcg, c->stream, nb, rho, nbt, true, true);
+    launch_cg_pass4_n(p, g, B.t, B.q, U, aee_of(c, p), op, B.rs, c->red, c->dcg, c->stream, nb, rho, nbt);
   } else {
     launch_mtil_pass1(p, g, false, B.t, B.p, U, ainv_of(c, p), op, c->dcg, c->stream, nb, kappa, AlphaFin{}, true);
-    launch_mtil_pass2(p, g, false, B.q, B.t, B.p, U, aee_of(c, p), op, c->red, nullptr, c->dcg, c->stream, nb, rho,
-                      kappa, true, true);
+    launch_mtil_pass2(p, g, false, B.q, B.t, B.p, U, aee_of(c, p), op, c->red, c->dcg, c->stream, nb, rho, kappa,
+                      true);
     launch_mtil_pass1(p, g, true, B.t, B.q, U, ainv_of(c, p), op, c->dcg, c->stream, nb, kappa, fin, true);
-    launch_cg_pass4(p, g, B.t, B.q, U, aee_of(c, p), op, B.rs, c->red, c->dcg, c->stream, nb, rho, kappa, true, true);
+    launch_cg_pass4(p, g, B.t, B.q, U, aee_of(c, p), op, B.rs, c->red, c->dcg, c->stream, nb, rho, kappa);
   }
 }
 
@@ -1106,8 +1106,8 @@ static int op_host(bqcdg_ctx* c, double* out, const double* in, const bqcdg_para
   if ((st = upload_spinor(c, in, si))) return st;
   OpParams op = op_of(p, which >= 3);
   switch (which) {
-    case 0: case 3: apply_mtil(c, Prec::F64, false, S(so), S(si), S(t), op, nullptr, nullptr); break;
-    case 1: case 4: apply_mtil(c, Prec::F64, true, S(so), S(si), S(t), op, nullptr, nullptr); break;
+    case 0: case 3: apply_mtil(c, Prec::F64, false, S(so), S(si), S(t), op); break;
+    case 1: case 4: apply_mtil(c, Prec::F64, true, S(so), S(si), S(t), op); break;
     default: apply_mdagm(c, Prec::F64, S(so), S(si), S(t), S(q), op);
   }
   CKL();

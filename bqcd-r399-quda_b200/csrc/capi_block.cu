@@ -263,11 +263,11 @@ extern "C" int bqcdg_solve_block(bqcdg_ctx* c, int nrhs, const int* hx, const in
       launch_mtil_pass1(Prec::F32, g, false, bs.T, bs.P, gauge_of(c, Prec::F32), ainv_of(c, Prec::F32), op,
                         nullptr, c->stream, s);
       launch_mtil_pass2(Prec::F32, g, false, bs.Qe, bs.T, bs.P, gauge_of(c, Prec::F32), aee_of(c, Prec::F32), op,
-                        c->red, nullptr, nullptr, c->stream, s);
+                        c->red, nullptr, c->stream, s);
       launch_mtil_pass1(Prec::F32, g, true, bs.T, bs.Qe, gauge_of(c, Prec::F32), ainv_of(c, Prec::F32), op,
                         nullptr, c->stream, s);
       launch_mtil_pass2(Prec::F32, g, true, bs.Z, bs.T, bs.Qe, gauge_of(c, Prec::F32), aee_of(c, Prec::F32), op,
-                        c->red, nullptr, nullptr, c->stream, s);
+                        c->red, nullptr, c->stream, s);
       CKL();
       Dense G, L;
       if ((st = gram(c, bs, s, bs.P, bs.Z, G))) return st;

@@ -174,8 +174,8 @@ int bqcdg_op_dev(bqcdg_ctx* c, int which, int hout, int hin, const bqcdg_params*
   OpParams op = op_of(p, which >= 3);
   SpinorPtr so = S(field(c, hout)), si = S(field(c, hin));
   switch (which) {
-    case 0: case 3: apply_mtil(c, Prec::F64, false, so, si, S(t), op, nullptr, nullptr); break;
-    case 1: case 4: apply_mtil(c, Prec::F64, true, so, si, S(t), op, nullptr, nullptr); break;
+    case 0: case 3: apply_mtil(c, Prec::F64, false, so, si, S(t), op); break;
+    case 1: case 4: apply_mtil(c, Prec::F64, true, so, si, S(t), op); break;
     default: apply_mdagm(c, Prec::F64, so, si, S(t), S(q), op);
   }
   CKL();

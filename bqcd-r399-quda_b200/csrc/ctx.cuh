@@ -200,7 +200,7 @@ CloverPtr aee_of(bqcdg_ctx* c, Prec p);
 CloverPtr ainv_of(bqcdg_ctx* c, Prec p);
 int check_op(bqcdg_ctx* c, const bqcdg_params* p);
 void apply_mtil(bqcdg_ctx* c, Prec p, bool dag, SpinorPtr out, SpinorPtr in, SpinorPtr t, const OpParams& op,
-                double* norm_out, CgScalars* cg, bool chain = false);
+                bool chain = false);
 void apply_mdagm(bqcdg_ctx* c, Prec p, SpinorPtr out, SpinorPtr in, SpinorPtr t, SpinorPtr q, const OpParams& op);
 int cg_core(bqcdg_ctx* c, double2* x, double2* b, const OpParams& op, Prec sloppy, int maxiter, double stop_rtr,
             double delta, bool min_one_iter, bool time_kernels, bqcdg_solve_info* info);

@@ -16,7 +16,7 @@ namespace bqcdg {
 // precision stencils move few bytes per thread, so latency hiding needs more
 // warps in flight than the FP64 ones (whose per-thread loads are 2-4x larger).
 // The second pass carries the clover block, the input spinor and (fused into
-// CG) x, r and p besides the hop, so it gets a larger register budget.
+// CG) r besides the hop, so it gets a larger register budget.
 #ifndef BQCDG_SLOPPY_MIN_BLOCKS
 #define BQCDG_SLOPPY_MIN_BLOCKS 6
 #endif
@@ -179,7 +179,7 @@ __global__ void __launch_bounds__(kBlock, Occ<P>::min_blocks) k_pass1(Geom g, Sp
   using R = typename SpinorView<P>::R;
   const Tile tl = tile(nr, fin.partial ? 1 : 0);
   if (tl.sb < 0) {
-    // alpha of the k_pass2 before (launched with defer_alpha): one CTA more
+    // alpha of the k_pass2 before (its block partials): one CTA more
     // per right-hand side, first in the launch
     chain_wait();
     double tot[1];
@@ -220,8 +220,8 @@ __global__ void __launch_bounds__(kBlock, Occ<P>::min_blocks) k_pass1(Geom g, Sp
 void launch_mtil_pass1(Prec p, const Geom& g, bool dag, SpinorPtr out_o, SpinorPtr in_e, const void* gauge,
                        CloverPtr ainv_oo, const OpParams& op, const CgScalars* cg, cudaStream_t s, int nr,
                        const double* kappa_rhs, AlphaFin fin, bool chain) {
-  if (split_sites(p, g) && !kappa_rhs) {
-    launch_split_pass1(g, dag, out_o, in_e, gauge, ainv_oo, op, cg, s, nr, fin, chain);
+  if (split_sites(p, g)) {
+    launch_split_pass1(g, dag, out_o, in_e, gauge, ainv_oo, op, cg, s, fin, chain);
     return;
   }
   dim3 grid((nblocks(g.volh) + (fin.partial ? 1 : 0)) * nr);
@@ -316,9 +316,8 @@ __device__ __forceinline__ void pass2_core(const Geom& g, int i, const SpinorVie
 template <Prec P, bool DAG, bool REDUCE, bool KT>
 __global__ void __launch_bounds__(kBlock, Occ<P>::min_blocks2) k_pass2(Geom g, SpinorPtr outp, SpinorPtr tp, SpinorPtr xp,
                                                   const void* gauge, CloverPtr aee, int has_clover, double bcoef,
-                                                  double hval, double rho, RedScratch red, double* norm_out,
-                                                  CgScalars* cg, int nr, const double* rho_rhs, double kappa,
-                                                  const double* kappa_rhs, bool defer_alpha) {
+                                                  double hval, double rho, RedScratch red, const CgScalars* cg, int nr,
+                                                  const double* rho_rhs, double kappa, const double* kappa_rhs) {
   using R = typename SpinorView<P>::R;
   const Tile tl = tile(nr);
   const CgScalars* me = cg ? cg + tl.rhs : nullptr;
@@ -349,51 +348,34 @@ __global__ void __launch_bounds__(kBlock, Occ<P>::min_blocks2) k_pass2(Geom g, S
   }
   if (REDUCE) {
     if (P == Prec::F16 && me && me->done) return;
-    double* part = red.partial + (size_t)tl.rhs * kRedVals * red.maxblocks;
-    block_reduce_store<1>(acc, part, red.maxblocks, tl.sb);
-    // defer_alpha: the partials stay for the next k_pass1 (AlphaFin).  The
-    // arrival counter of the last-block sum costs a k_pass2<int16> at 32^3x64
-    // 8 % of its time (137 against 127 us), its partial stores alone nothing.
-    if (!defer_alpha && last_block(red.counter + tl.rhs, tl.nsb)) {
-      double tot[1];
-      final_sum<1>(part, red.maxblocks, tl.nsb, tot);
-      if (threadIdx.x == 0) {
-        if (norm_out) norm_out[tl.rhs] = tot[0];
-        if (cg) {
-          cg_set_alpha(cg + tl.rhs, tot[0]);
-        }
-        red.counter[tl.rhs] = 0;
-      }
-    }
+    block_reduce_store<1>(acc, red.partial + (size_t)tl.rhs * kRedVals * red.maxblocks, red.maxblocks, tl.sb);
+    // The sum is left to the next k_pass1 (AlphaFin): an arrival counter
+    // here costs a k_pass2<int16> at 32^3x64 8 % of its time (137 against 127
+    // us), the partial stores alone nothing.
   }
 }
 
 void launch_mtil_pass2(Prec p, const Geom& g, bool dag, SpinorPtr out_e, SpinorPtr t_o, SpinorPtr in_e,
-                       const void* gauge, CloverPtr a_ee, const OpParams& op, RedScratch red, double* norm_out,
-                       CgScalars* cg, cudaStream_t s, int nr, const double* rho_rhs, const double* kappa_rhs,
-                       bool defer_alpha, bool chain) {
+                       const void* gauge, CloverPtr a_ee, const OpParams& op, RedScratch red, const CgScalars* cg,
+                       cudaStream_t s, int nr, const double* rho_rhs, const double* kappa_rhs, bool chain) {
   dim3 grid(nblocks(g.volh) * nr);
   int hc = op.csw_kappa != 0.0;
   double bcoef = -op.kappa * op.kappa / (1.0 + op.h * op.h);
   double hv = dag ? -op.h : op.h;
-  bool reduce = norm_out != nullptr || cg != nullptr;
-  defer_alpha = defer_alpha && cg && !norm_out;  // only alpha can wait for the next pass
-  if (split_sites(p, g) && !kappa_rhs && (defer_alpha || !reduce)) {
-    launch_split_pass2(g, dag, out_e, t_o, in_e, gauge, a_ee, op, red, reduce, cg, s, nr, rho_rhs, chain);
+  const bool reduce = cg != nullptr;  // never with dag, whose CG pass is k_cg_pass4
+  if (split_sites(p, g)) {
+    launch_split_pass2(g, dag, out_e, t_o, in_e, gauge, a_ee, op, red, cg, s, chain);
     return;
   }
 #define P2(PP, D, RR, K)                                                                                        \
   launch_chain(chain, k_pass2<PP, D, RR, K>, grid, kBlock, s, g, out_e, t_o, in_e, gauge, a_ee, hc, bcoef, hv, op.rho, \
-               red, norm_out, cg, nr, rho_rhs, op.kappa, kappa_rhs, defer_alpha)
-#define P2R(PP, D)                                         \
-  if (g.clover_t) {                                        \
-    if (reduce) P2(PP, D, true, true); else P2(PP, D, false, true);   \
-  } else {                                                 \
-    if (reduce) P2(PP, D, true, false); else P2(PP, D, false, false); \
-  }
-  if (p == Prec::F64) { if (dag) { P2R(Prec::F64, true) } else { P2R(Prec::F64, false) } }
-  else if (p == Prec::F32) { if (dag) { P2R(Prec::F32, true) } else { P2R(Prec::F32, false) } }
-  else { if (dag) { P2R(Prec::F16, true) } else { P2R(Prec::F16, false) } }
+               red, cg, nr, rho_rhs, op.kappa, kappa_rhs)
+#define P2R(PP, D, RR) if (g.clover_t) P2(PP, D, RR, true); else P2(PP, D, RR, false);
+#define P2D(PP) if (reduce) { P2R(PP, false, true) } else if (dag) { P2R(PP, true, false) } else { P2R(PP, false, false) }
+  if (p == Prec::F64) { P2D(Prec::F64) }
+  else if (p == Prec::F32) { P2D(Prec::F32) }
+  else { P2D(Prec::F16) }
+#undef P2D
 #undef P2R
 #undef P2
 }
@@ -401,27 +383,16 @@ void launch_mtil_pass2(Prec p, const Geom& g, bool dag, SpinorPtr out_e, SpinorP
 // ---------------------------------------------------------------------------
 // CG-fused last pass of M^+M (cg.F90:93-107 folded into mtil_dag's second half)
 // ---------------------------------------------------------------------------
-template <Prec XP>
-struct XR;
-template <>
-struct XR<Prec::F64> {
-  using View = SpinorView<Prec::F64>;
-};
-template <>
-struct XR<Prec::F32> {
-  using View = SpinorView<Prec::F32>;
-};
-
 template <Prec P, Prec XP, bool KT>
 __global__ void __launch_bounds__(kBlock, Occ<P>::min_blocks2) k_cg_pass4(Geom g, SpinorPtr tp, SpinorPtr qp, const void* gauge,
                                                      CloverPtr aee, int has_clover, double bcoef, double hval,
                                                      double rho, SpinorPtr rp,
-                                                     RedScratch red, CgScalars* cgs, int nr, const double* rho_rhs,
-                                                     double kappa, const double* kappa_rhs, bool defer_step) {
+                                                     RedScratch red, const CgScalars* cgs, int nr,
+                                                     const double* rho_rhs, double kappa, const double* kappa_rhs) {
   using R = typename SpinorView<P>::R;
   using RX = typename SpinorView<XP>::R;
   const Tile tl = tile(nr);
-  CgScalars* cg = cgs + tl.rhs;
+  const CgScalars* cg = cgs + tl.rhs;
   if (idle<P>(cg)) return;
   if (rho_rhs) rho = rho_rhs[tl.rhs];  // a shift per right-hand side
   if (kappa_rhs) {                      // a hopping parameter per right-hand side
@@ -453,19 +424,10 @@ __global__ void __launch_bounds__(kBlock, Occ<P>::min_blocks2) k_cg_pass4(Geom g
     chain_wait();
     if (P == Prec::F16 && cg->done) return;
   }
-  double* part = red.partial + (size_t)tl.rhs * kRedVals * red.maxblocks;
-  block_reduce_store<1>(acc, part, red.maxblocks, tl.sb);
-  if (!defer_step && last_block(red.counter + tl.rhs, tl.nsb)) {
-    double tot[1];
-    final_sum<1>(part, red.maxblocks, tl.nsb, tot);
-    if (threadIdx.x == 0) {
-      cg_scalar_step(cg, tot[0]);
-      red.counter[tl.rhs] = 0;
-    }
-  }
+  block_reduce_store<1>(acc, red.partial + (size_t)tl.rhs * kRedVals * red.maxblocks, red.maxblocks, tl.sb);
 }
 
-// the deferred step of k_cg_pass4 (defer_step): CTA r sums RHS r's partials
+// the step of k_cg_pass4's iteration: CTA r sums RHS r's partials
 // with all its threads in flight at once and steps its scalars
 constexpr int kStepBlock = 1024;
 __global__ void __launch_bounds__(kStepBlock) k_cg_step(RedScratch red, CgScalars* cgs, int nsb) {
@@ -482,10 +444,10 @@ void launch_cg_step(RedScratch red, CgScalars* cg, int nr, int nsb, cudaStream_t
 }
 
 void launch_cg_pass4(Prec p, const Geom& g, SpinorPtr t_o, SpinorPtr q_e, const void* gauge, CloverPtr a_ee,
-                     const OpParams& op, SpinorPtr r, RedScratch red, CgScalars* cg, cudaStream_t s, int nr,
-                     const double* rho_rhs, const double* kappa_rhs, bool defer_step, bool chain) {
-  if (split_sites(p, g) && !kappa_rhs && defer_step) {
-    launch_split_pass4(g, t_o, q_e, gauge, a_ee, op, r, red, cg, s, nr, rho_rhs, chain);
+                     const OpParams& op, SpinorPtr r, RedScratch red, const CgScalars* cg, cudaStream_t s, int nr,
+                     const double* rho_rhs, const double* kappa_rhs) {
+  if (split_sites(p, g)) {
+    launch_split_pass4(g, t_o, q_e, gauge, a_ee, op, r, red, cg, s);
     return;
   }
   dim3 grid(nblocks(g.volh) * nr);
@@ -493,8 +455,8 @@ void launch_cg_pass4(Prec p, const Geom& g, SpinorPtr t_o, SpinorPtr q_e, const 
   double bcoef = -op.kappa * op.kappa / (1.0 + op.h * op.h);
   double hv = -op.h;  // mtil_dag
 #define P4(PP, XX, K)                                                                                             \
-  launch_chain(chain, k_cg_pass4<PP, XX, K>, grid, kBlock, s, g, t_o, q_e, gauge, a_ee, hc, bcoef, hv, op.rho, r, red, \
-               cg, nr, rho_rhs, op.kappa, kappa_rhs, defer_step)
+  launch_chain(true, k_cg_pass4<PP, XX, K>, grid, kBlock, s, g, t_o, q_e, gauge, a_ee, hc, bcoef, hv, op.rho, r, red, \
+               cg, nr, rho_rhs, op.kappa, kappa_rhs)
 #define P4K(PP, XX) if (g.clover_t) P4(PP, XX, true); else P4(PP, XX, false);
   if (p == Prec::F64) { P4K(Prec::F64, Prec::F64) }
   else if (p == Prec::F32) { P4K(Prec::F32, Prec::F32) }

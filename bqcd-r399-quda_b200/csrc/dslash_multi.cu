@@ -202,7 +202,7 @@ __global__ void __launch_bounds__(kBlock, OccN<NB>::min_blocks)
   chain_wait();
   if (!group_live<NB>(cg, rhs0, nr, act)) return;
   if (tl.sb < 0) {
-    // alpha of the k_pass2_n before (defer_alpha), as in k_pass1
+    // alpha of the k_pass2_n before, as in k_pass1
     double tot[NB];
     final_sum<NB>(after_wait(fin.partial) + (size_t)rhs0 * kRedVals * fin.stride, kRedVals * fin.stride, tl.nsb, tot);
     if (threadIdx.x == 0) {
@@ -313,13 +313,12 @@ __device__ __forceinline__ void group_rho(double rho, const double* rho_rhs, int
   for (int r = 0; r < NB; r++) out[r] = rho_rhs && act[r] ? rho_rhs[rhs0 + r] : rho;
 }
 
-// q_r = M~ p_r (second half, dag = false) with the CG alpha_r = rtr_r /
-// |q_r|^2 of every live RHS (k_pass2 of dslash.cu with its reduction)
+// q_r = M~ p_r (second half, dag = false) with the |q_r|^2 block partials of
+// every live RHS (k_pass2 of dslash.cu with its reduction)
 template <Prec P, int NB>
 __global__ void __launch_bounds__(kBlock, OccN<NB>::min_blocks)
     k_pass2_n(Geom g, SpinorPtr outp, SpinorPtr tp, SpinorPtr xp, const void* gauge, CloverPtr aee, int has_clover,
-              double bcoef, double rho, RedScratch red, CgScalars* cg, int nr, int ng, const double* rho_rhs,
-              bool defer_alpha) {
+              double bcoef, double rho, RedScratch red, const CgScalars* cg, int nr, int ng, const double* rho_rhs) {
   using R = typename SpinorView<P>::R;
   const GTile tl = gtile(ng);
   const int rhs0 = tl.grp * NB;
@@ -352,44 +351,32 @@ __global__ void __launch_bounds__(kBlock, OccN<NB>::min_blocks)
     }
   }
   // value r of the group goes to the partial slot of RHS rhs0 + r
-  double* part = red.partial + (size_t)rhs0 * kRedVals * red.maxblocks;
-  block_reduce_store<NB>(acc, part, kRedVals * red.maxblocks, tl.sb);
-  if (!defer_alpha && last_block(red.counter + rhs0, tl.nsb)) {
-    double tot[NB];
-    final_sum<NB>(part, kRedVals * red.maxblocks, tl.nsb, tot);
-    if (threadIdx.x == 0) {
-#pragma unroll
-      for (int r = 0; r < NB; r++) {
-        if (!act[r]) continue;
-        cg_set_alpha(cg + rhs0 + r, tot[r]);
-      }
-      red.counter[rhs0] = 0;
-    }
-  }
+  block_reduce_store<NB>(acc, red.partial + (size_t)rhs0 * kRedVals * red.maxblocks, kRedVals * red.maxblocks, tl.sb);
 }
 
 void launch_mtil_pass2_n(Prec p, const Geom& g, SpinorPtr out_e, SpinorPtr t_o, SpinorPtr in_e, const void* gauge,
-                         CloverPtr a_ee, const OpParams& op, RedScratch red, CgScalars* cg, cudaStream_t s, int nr,
-                         const double* rho_rhs, int nbt, bool defer_alpha, bool chain) {
+                         CloverPtr a_ee, const OpParams& op, RedScratch red, const CgScalars* cg, cudaStream_t s,
+                         int nr, const double* rho_rhs, int nbt) {
   const int ng = (nr + nbt - 1) / nbt;
   dim3 grid(nblocks(g.volh) * ng);
   int hc = op.csw_kappa != 0.0;
   double bcoef = -op.kappa * op.kappa;  // h = 0
 #define P2N(PP, N)                                                                                          \
-  launch_chain(chain, k_pass2_n<PP, N>, grid, kBlock, s, g, out_e, t_o, in_e, gauge, a_ee, hc, bcoef, op.rho, red, \
-               cg, nr, ng, rho_rhs, defer_alpha)
+  launch_chain(true, k_pass2_n<PP, N>, grid, kBlock, s, g, out_e, t_o, in_e, gauge, a_ee, hc, bcoef, op.rho, red, \
+               cg, nr, ng, rho_rhs)
   if (p == Prec::F32) { if (nbt == 2) P2N(Prec::F32, 2); else P2N(Prec::F32, 4); }
   else { if (nbt == 2) P2N(Prec::F16, 2); else P2N(Prec::F16, 4); }
 #undef P2N
 }
 
 // CG-fused second half of mtil_dag for NB right-hand sides (k_cg_pass4 of
-// dslash.cu): Ap_r = A_ee q_r + b D_eo t_r + rho_r q_r, r_r -= alpha_r Ap_r, and the CG scalars from |r_r|^2
+// dslash.cu): Ap_r = A_ee q_r + b D_eo t_r + rho_r q_r, r_r -= alpha_r Ap_r, and the
+// |r_r|^2 block partials
 template <Prec P, int NB>
 __global__ void __launch_bounds__(kBlock, OccN<NB>::min_blocks)
     k_cg_pass4_n(Geom g, SpinorPtr tp, SpinorPtr qp, const void* gauge, CloverPtr aee, int has_clover, double bcoef,
-                 double rho, SpinorPtr rp, RedScratch red, CgScalars* cgs, int nr, int ng,
-                 const double* rho_rhs, bool defer_step) {
+                 double rho, SpinorPtr rp, RedScratch red, const CgScalars* cgs, int nr, int ng,
+                 const double* rho_rhs) {
   using R = typename SpinorView<P>::R;
   const GTile tl = gtile(ng);
   const int rhs0 = tl.grp * NB;
@@ -428,32 +415,19 @@ __global__ void __launch_bounds__(kBlock, OccN<NB>::min_blocks)
       rv.store(i, rl);
     }
   }
-  double* part = red.partial + (size_t)rhs0 * kRedVals * red.maxblocks;
-  block_reduce_store<NB>(acc, part, kRedVals * red.maxblocks, tl.sb);
-  if (!defer_step && last_block(red.counter + rhs0, tl.nsb)) {
-    double tot[NB];
-    final_sum<NB>(part, kRedVals * red.maxblocks, tl.nsb, tot);
-    if (threadIdx.x == 0) {
-#pragma unroll
-      for (int r = 0; r < NB; r++) {
-        if (!act[r]) continue;
-        cg_scalar_step(cgs + rhs0 + r, tot[r]);
-      }
-      red.counter[rhs0] = 0;
-    }
-  }
+  block_reduce_store<NB>(acc, red.partial + (size_t)rhs0 * kRedVals * red.maxblocks, kRedVals * red.maxblocks, tl.sb);
 }
 
 void launch_cg_pass4_n(Prec p, const Geom& g, SpinorPtr t_o, SpinorPtr q_e, const void* gauge, CloverPtr a_ee,
-                       const OpParams& op, SpinorPtr r, RedScratch red, CgScalars* cg, cudaStream_t s, int nr,
-                       const double* rho_rhs, int nbt, bool defer_step, bool chain) {
+                       const OpParams& op, SpinorPtr r, RedScratch red, const CgScalars* cg, cudaStream_t s, int nr,
+                       const double* rho_rhs, int nbt) {
   const int ng = (nr + nbt - 1) / nbt;
   dim3 grid(nblocks(g.volh) * ng);
   int hc = op.csw_kappa != 0.0;
   double bcoef = -op.kappa * op.kappa;  // h = 0
 #define P4N(PP, N)                                                                                              \
-  launch_chain(chain, k_cg_pass4_n<PP, N>, grid, kBlock, s, g, t_o, q_e, gauge, a_ee, hc, bcoef, op.rho, r, red, cg, \
-               nr, ng, rho_rhs, defer_step)
+  launch_chain(true, k_cg_pass4_n<PP, N>, grid, kBlock, s, g, t_o, q_e, gauge, a_ee, hc, bcoef, op.rho, r, red, cg, \
+               nr, ng, rho_rhs)
   if (p == Prec::F32) { if (nbt == 2) P4N(Prec::F32, 2); else P4N(Prec::F32, 4); }
   else { if (nbt == 2) P4N(Prec::F16, 2); else P4N(Prec::F16, 4); }
 #undef P4N

@@ -84,8 +84,7 @@ enum class Pass { First, Second, SecondSum, Cg };
 template <bool DAG, Pass W>
 __global__ void __launch_bounds__(128, 3)
     k_split(Geom g, SpinorPtr outp, SpinorPtr tp, SpinorPtr xp, const void* gauge, CloverPtr ap, int has_clover,
-            double bcoef, double hval, double rho, RedScratch red, const CgScalars* cgs, int nr, const double* rho_rhs,
-            AlphaFin fin) {
+            double bcoef, double hval, double rho, RedScratch red, const CgScalars* cg, AlphaFin fin) {
   using R = double;
   using R2 = double2;
   constexpr Prec P = Prec::F64;
@@ -95,27 +94,26 @@ __global__ void __launch_bounds__(128, 3)
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int chi = warp >> 1, s = warp & 1;
   const int extra = fin.partial ? 1 : 0;
-  const int rhs = blockIdx.x % nr, sb = (int)(blockIdx.x / nr) - extra, nsb = gridDim.x / nr - extra;
+  const int sb = (int)blockIdx.x - extra, nsb = (int)gridDim.x - extra;
   if (sb < 0) {
     // alpha of the second pass before (k_pass1's extra CTA)
     chain_wait();
     double tot[1];
-    final_sum<1>(after_wait(fin.partial) + (size_t)rhs * kRedVals * fin.stride, fin.stride, nsb, tot);
-    if (threadIdx.x == 0 && !fin.cg[rhs].done) cg_set_alpha(fin.cg + rhs, tot[0]);
+    final_sum<1>(after_wait(fin.partial), fin.stride, nsb, tot);
+    if (threadIdx.x == 0 && !fin.cg->done) cg_set_alpha(fin.cg, tot[0]);
     return;
   }
-  if (retired(cgs ? cgs + rhs : nullptr)) return;
+  if (retired(cg)) return;
   // threads beyond the last site work on it too, and store nothing
   const int i0 = sb * kSplitSites + lane;
   const bool live = i0 < g.volh;
   const int i = live ? i0 : g.volh - 1;
-  if (rho_rhs) rho = rho_rhs[rhs];
   const auto U = gview<P>(gauge, g);
   const Site st = site_coords(g, i, e);
 
   chain_wait();
-  const bool stopped = cgs && cgs[rhs].done;
-  const auto t = after_wait(sview<P>(rhs_of(tp, rhs), g.stride));
+  const bool stopped = cg && cg->done;
+  const auto t = after_wait(sview<P>(tp, g.stride));
   Spinor<R> b;
   zero(b);
   const R hs = W == Pass::First ? 1.0 : bcoef;
@@ -136,7 +134,7 @@ __global__ void __launch_bounds__(128, 3)
   if constexpr (W != Pass::First) {
     // the site-local terms: rows of A_ee x and of rho x
     Spinor<R> x;
-    after_wait(sview<P>(rhs_of(xp, rhs), g.stride)).load(i, x);
+    after_wait(sview<P>(xp, g.stride)).load(i, x);
     cx<R> xc[6];
 #pragma unroll
     for (int k = 0; k < 6; k++)
@@ -195,9 +193,9 @@ __global__ void __launch_bounds__(128, 3)
   }
   const int sp = s + 2 * chi;
   double acc[1] = {0.0};
-  const auto out = after_wait(sview<P>(rhs_of(outp, rhs), g.stride));
+  const auto out = after_wait(sview<P>(outp, g.stride));
   if (W == Pass::Cg) {
-    const R al = cgs[rhs].alpha;  // set by the launch before
+    const R al = cg->alpha;  // set by the launch before
 #pragma unroll
     for (int c = 0; c < 3; c++) {
       const double2 r = ld_field(out.v + (c * 4 + sp) * out.stride + i);
@@ -211,42 +209,41 @@ __global__ void __launch_bounds__(128, 3)
   }
   if (W == Pass::SecondSum || W == Pass::Cg) {
     if (!live) acc[0] = 0.0;
-    block_reduce_store<1>(acc, red.partial + (size_t)rhs * kRedVals * red.maxblocks, red.maxblocks, sb);
+    block_reduce_store<1>(acc, red.partial, red.maxblocks, sb);
   }
 }
 
 void launch_split_pass1(const Geom& g, bool dag, SpinorPtr out, SpinorPtr in, const void* gauge, CloverPtr a,
-                        const OpParams& op, const CgScalars* cg, cudaStream_t s, int nr, AlphaFin fin, bool chain) {
-  const dim3 grid((site_blocks(Prec::F64, g) + (fin.partial ? 1 : 0)) * nr);
+                        const OpParams& op, const CgScalars* cg, cudaStream_t s, AlphaFin fin, bool chain) {
+  const dim3 grid(site_blocks(Prec::F64, g) + (fin.partial ? 1 : 0));
   const int hc = op.csw_kappa != 0.0;
   const double hv = dag ? op.h : -op.h;
 #define SP1(D)                                                                                              \
   launch_chain(chain, k_split<D, Pass::First>, grid, 128, s, g, out, in, SpinorPtr{}, gauge, a, hc, 0.0, hv, 0.0, \
-               RedScratch{}, cg, nr, nullptr, fin)
+               RedScratch{}, cg, fin)
   if (dag) SP1(true); else SP1(false);
 #undef SP1
 }
 
 void launch_split_pass2(const Geom& g, bool dag, SpinorPtr out, SpinorPtr t, SpinorPtr x, const void* gauge,
-                        CloverPtr a, const OpParams& op, RedScratch red, bool sum, const CgScalars* cg,
-                        cudaStream_t s, int nr, const double* rho_rhs, bool chain) {
-  const dim3 grid(site_blocks(Prec::F64, g) * nr);
+                        CloverPtr a, const OpParams& op, RedScratch red, const CgScalars* cg, cudaStream_t s,
+                        bool chain) {
+  const dim3 grid(site_blocks(Prec::F64, g));
   const int hc = op.csw_kappa != 0.0;
   const double bcoef = -op.kappa * op.kappa / (1.0 + op.h * op.h), hv = dag ? -op.h : op.h;
-#define SP2(D, W)                                                                                             \
-  launch_chain(chain, k_split<D, W>, grid, 128, s, g, out, t, x, gauge, a, hc, bcoef, hv, op.rho, red, cg, nr, \
-               rho_rhs, AlphaFin{})
-  if (sum) { if (dag) SP2(true, Pass::SecondSum); else SP2(false, Pass::SecondSum); }
-  else { if (dag) SP2(true, Pass::Second); else SP2(false, Pass::Second); }
+#define SP2(D, W)                                                                                                   \
+  launch_chain(chain, k_split<D, W>, grid, 128, s, g, out, t, x, gauge, a, hc, bcoef, hv, op.rho, red, cg, AlphaFin{})
+  if (cg) SP2(false, Pass::SecondSum);
+  else if (dag) SP2(true, Pass::Second);
+  else SP2(false, Pass::Second);
 #undef SP2
 }
 
 void launch_split_pass4(const Geom& g, SpinorPtr t, SpinorPtr q, const void* gauge, CloverPtr a, const OpParams& op,
-                        SpinorPtr r, RedScratch red, const CgScalars* cg, cudaStream_t s, int nr,
-                        const double* rho_rhs, bool chain) {
+                        SpinorPtr r, RedScratch red, const CgScalars* cg, cudaStream_t s) {
   const double bcoef = -op.kappa * op.kappa / (1.0 + op.h * op.h);
-  launch_chain(chain, k_split<true, Pass::Cg>, dim3(site_blocks(Prec::F64, g) * nr), 128, s, g, r, t, q, gauge, a,
-               (int)(op.csw_kappa != 0.0), bcoef, -op.h, op.rho, red, cg, nr, rho_rhs, AlphaFin{});
+  launch_chain(true, k_split<true, Pass::Cg>, dim3(site_blocks(Prec::F64, g)), 128, s, g, r, t, q, gauge, a,
+               (int)(op.csw_kappa != 0.0), bcoef, -op.h, op.rho, red, cg, AlphaFin{});
 }
 
 }  // namespace bqcdg

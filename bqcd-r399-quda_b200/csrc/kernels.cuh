@@ -101,75 +101,71 @@ void launch_clover_mult(Prec p, const Geom& g, SpinorPtr out, SpinorPtr in, Clov
 // in-place LDL solve with the B factors (F64 only)
 void launch_clover_mult_b(const Geom& g, double2* x, const double2* b, cudaStream_t s);
 
-// first half of mtil / mtil_dag: out_o = [(1 -+ i h g5)] Ainv_oo D_oe in_e
-// (nr > 1: nr right-hand sides in one launch, fields at SpinorPtr::rsb strides,
-//  cg / norm_out arrays of nr entries; retired RHS return at once)
-// (g.clover_t: the clover fields hold T and each pass forms A(kappa) and
-//  A(kappa)^-1 per site, at op.kappa or at kappa_rhs[k] for right-hand side k;
-//  kappa_rhs also sets each right-hand side's hopping coefficient)
-// The |M~ p|^2 block partials that a k_pass2 launched with defer_alpha left
-// in red.partial (slot 0 of each RHS).  The k_pass1 launch after it, given
-// this, sums them in one more CTA per RHS and sets that RHS's paap and alpha = rtr / paap: the same fixed-order sum
-// (final_sum) that k_pass2's last block would run, so alpha is bit for bit
-// the same, but no k_pass2 block waits for an arrival counter.
+// The passes of an operator or a CG iteration.  nr > 1 (FP32 and int16): nr
+// right-hand sides in one launch, fields at SpinorPtr::rsb strides, cg an array
+// of nr entries; a retired one returns at once.  g.clover_t: the clover fields
+// hold T and each pass forms A(kappa) and A(kappa)^-1 per site, at op.kappa or
+// at kappa_rhs[k] for right-hand side k, which also sets its hopping
+// coefficient.  rho_rhs: one shift per right-hand side (device), in place of
+// op.rho in the second passes.
+//
+// The |M~ p|^2 block partials that a second pass with cg left in red.partial
+// (slot 0 of each RHS).  The k_pass1 launch after it, given this, sums them in
+// one more CTA per RHS (final_sum) and sets that RHS's paap and alpha = rtr /
+// paap, so no CTA of the second pass waits for an arrival counter.
 struct AlphaFin {
   const double* partial = nullptr;
   int stride = 0;  // RedScratch::maxblocks
   CgScalars* cg = nullptr;
 };
+// first half of mtil / mtil_dag: out_o = [(1 -+ i h g5)] Ainv_oo D_oe in_e
 void launch_mtil_pass1(Prec p, const Geom& g, bool dag, SpinorPtr out_o, SpinorPtr in_e, const void* gauge,
                        CloverPtr ainv_oo, const OpParams& op, const CgScalars* cg, cudaStream_t s, int nr = 1,
                        const double* kappa_rhs = nullptr, AlphaFin fin = AlphaFin{}, bool chain = false);
 // second half: out_e = A_ee in_e + b D_eo t_o (+ h term for Wilson) + rho in_e;
-// optional |out|^2 reduction into *norm_out (device), and CG alpha update
+// with cg (dag = false only) also the |out|^2 block partials
 void launch_mtil_pass2(Prec p, const Geom& g, bool dag, SpinorPtr out_e, SpinorPtr t_o, SpinorPtr in_e,
-                       const void* gauge, CloverPtr a_ee, const OpParams& op, RedScratch red, double* norm_out,
-                       CgScalars* cg, cudaStream_t s, int nr = 1, const double* rho_rhs = nullptr,
-                       const double* kappa_rhs = nullptr, bool defer_alpha = false, bool chain = false);
+                       const void* gauge, CloverPtr a_ee, const OpParams& op, RedScratch red, const CgScalars* cg,
+                       cudaStream_t s, int nr = 1, const double* rho_rhs = nullptr, const double* kappa_rhs = nullptr,
+                       bool chain = false);
 // CG-fused second half of mtil_dag: Ap = A_ee q + b D_eo t_o + rho q computed in
-// registers; r -= alpha Ap, rtr = |r|^2 (x += alpha p follows in
-// k_cg_pupdate).  Precision P for the stencil fields, r in XP (F64 for the FP64 solver, F32 for the sloppy one)
+// registers; r -= alpha Ap and the |r|^2 block partials (x += alpha p follows in
+// k_cg_pupdate).  Precision P for the stencil fields, r in XP (F64 for the FP64
+// solver, F32 for the sloppy one)
 void launch_cg_pass4(Prec p, const Geom& g, SpinorPtr t_o, SpinorPtr q_e, const void* gauge, CloverPtr a_ee,
-                     const OpParams& op, SpinorPtr r, RedScratch red, CgScalars* cg, cudaStream_t s, int nr = 1,
-                     const double* rho_rhs = nullptr, const double* kappa_rhs = nullptr, bool defer_step = false,
-                     bool chain = false);
-// With defer_step, k_cg_pass4 leaves its |r|^2 block partials in red.partial
-// and launch_cg_step, queued after it, sums them (one CTA per right-hand
-// side, the fixed-order final_sum) and takes the CG scalar step
-// (cg_scalar_step: beta, the stop tests), which the last k_cg_pass4 block
-// would otherwise take after an arrival counter.  nsb: site blocks per RHS
-// of that k_cg_pass4 launch.
+                     const OpParams& op, SpinorPtr r, RedScratch red, const CgScalars* cg, cudaStream_t s, int nr = 1,
+                     const double* rho_rhs = nullptr, const double* kappa_rhs = nullptr);
+// queued after it: sums the |r|^2 partials (one CTA per right-hand side, the
+// fixed-order final_sum) and takes the CG scalar step (cg_scalar_step: beta, the
+// stop tests).  nsb: site blocks per RHS of that k_cg_pass4 launch.
 void launch_cg_step(RedScratch red, CgScalars* cg, int nr, int nsb, cudaStream_t s);
-// (rho_rhs: device array of one shift rho per right-hand side, replacing
-//  op.rho, in the second passes; null: op.rho for all)
 // register-blocked batched passes (dslash_multi.cu): one thread serves one
 // site of nbt (2 or 4) right-hand sides, so each link and clover block is
 // loaded and decoded once for all of them.  Sloppy precisions (F32, F16)
-// and h = 0 only; pass 2 is the non-dagger one with the CG alpha update (cg
+// and h = 0 only; pass 2 is the non-dagger one with its block partials (cg
 // required there and in pass 4).
 void launch_mtil_pass1_n(Prec p, const Geom& g, bool dag, SpinorPtr out_o, SpinorPtr in_e, const void* gauge,
                          CloverPtr ainv_oo, const OpParams& op, const CgScalars* cg, cudaStream_t s, int nr,
                          int nbt, AlphaFin fin = AlphaFin{}, bool chain = false);
 void launch_mtil_pass2_n(Prec p, const Geom& g, SpinorPtr out_e, SpinorPtr t_o, SpinorPtr in_e, const void* gauge,
-                         CloverPtr a_ee, const OpParams& op, RedScratch red, CgScalars* cg, cudaStream_t s, int nr,
-                         const double* rho_rhs, int nbt, bool defer_alpha = false, bool chain = false);
+                         CloverPtr a_ee, const OpParams& op, RedScratch red, const CgScalars* cg, cudaStream_t s,
+                         int nr, const double* rho_rhs, int nbt);
 void launch_cg_pass4_n(Prec p, const Geom& g, SpinorPtr t_o, SpinorPtr q_e, const void* gauge, CloverPtr a_ee,
-                       const OpParams& op, SpinorPtr r, RedScratch red, CgScalars* cg, cudaStream_t s, int nr,
-                       const double* rho_rhs, int nbt, bool defer_step = false, bool chain = false);
+                       const OpParams& op, SpinorPtr r, RedScratch red, const CgScalars* cg, cudaStream_t s, int nr,
+                       const double* rho_rhs, int nbt);
 // the same three passes of FP64 fields with four threads per site
 // (dslash_split.cu), which the launchers above take where split_sites says so:
-// stored clover blocks, one kappa, deferred sums.  site_blocks: the block
-// partials of a pass, at most kRedVals maxblocks per right-hand side
+// one right-hand side, stored clover blocks.  site_blocks: the block partials
+// of a pass, at most kRedVals maxblocks
 bool split_sites(Prec p, const Geom& g);
 int site_blocks(Prec p, const Geom& g);
 void launch_split_pass1(const Geom& g, bool dag, SpinorPtr out, SpinorPtr in, const void* gauge, CloverPtr a,
-                        const OpParams& op, const CgScalars* cg, cudaStream_t s, int nr, AlphaFin fin, bool chain);
+                        const OpParams& op, const CgScalars* cg, cudaStream_t s, AlphaFin fin, bool chain);
 void launch_split_pass2(const Geom& g, bool dag, SpinorPtr out, SpinorPtr t, SpinorPtr x, const void* gauge,
-                        CloverPtr a, const OpParams& op, RedScratch red, bool sum, const CgScalars* cg,
-                        cudaStream_t s, int nr, const double* rho_rhs, bool chain);
+                        CloverPtr a, const OpParams& op, RedScratch red, const CgScalars* cg, cudaStream_t s,
+                        bool chain);
 void launch_split_pass4(const Geom& g, SpinorPtr t, SpinorPtr q, const void* gauge, CloverPtr a, const OpParams& op,
-                        SpinorPtr r, RedScratch red, const CgScalars* cg, cudaStream_t s, int nr,
-                        const double* rho_rhs, bool chain);
+                        SpinorPtr r, RedScratch red, const CgScalars* cg, cudaStream_t s);
 // p = r + beta p, and the x += alpha p of iteration expect.n[rhs] if that
 // iteration ran
 void launch_cg_pupdate(Prec p, const Geom& g, SpinorPtr pvec, SpinorPtr r, CgScalars* cg, cudaStream_t s,

@@ -76,8 +76,8 @@ extern "C" int bqcdg_mdagm_noalloc(const int L[4], const int bc[4], const double
   // every site these passes read is written first, so nothing in the scratch
   // has to start at zero
   launch_mtil_pass1(Prec::F64, g, false, t, si, gauge, aio, op, nullptr, s);
-  launch_mtil_pass2(Prec::F64, g, false, q, t, si, gauge, aee, op, none, nullptr, nullptr, s);
+  launch_mtil_pass2(Prec::F64, g, false, q, t, si, gauge, aee, op, none, nullptr, s);
   launch_mtil_pass1(Prec::F64, g, true, t, q, gauge, aio, op, nullptr, s);
-  launch_mtil_pass2(Prec::F64, g, true, so, t, q, gauge, aee, op, none, nullptr, nullptr, s);
+  launch_mtil_pass2(Prec::F64, g, true, so, t, q, gauge, aee, op, none, nullptr, s);
   return cudaGetLastError() == cudaSuccess ? BQCDG_OK : BQCDG_ECUDA;
 }
