@@ -4,12 +4,16 @@
 // The passes of dslash.cu give a site one thread: a chain of eight hops, each
 // a round of loads and about 250 instructions, then the clover blocks.  On a
 // lattice that leaves most of the GPU idle that chain is the time of the pass,
-// 7 us at 8^4.  Here a
-// CTA of four warps serves 32 sites (lane = site).  Warp mu forms the two hops
-// of direction mu, the partial sums meet in shared memory, and warp (chi, s)
-// then forms rows 3s..3s+2 of chiral block chi and the spin s + 2 chi of the
-// result.  Everything stays in the chiral basis x+- = up +- dn, in which the
-// clover blocks and the h terms are diagonal, until the last exchange.
+// 7 us at 8^4.  Here a CTA of four warps serves 32 sites (lane = site).  Warp
+// mu forms the two hops of direction mu, the partial sums meet in shared
+// memory, and warp (chi, s) then forms rows 3s..3s+2 of chiral block chi and the
+// spin s + 2 chi of the result.  Everything stays in the chiral basis x+- = up
+// +- dn, in which the clover blocks and the h terms are diagonal, until the last
+// exchange.  So the Wilson and rho terms of a spin, which the one-thread passes
+// add to that spin alone, come back from the sum and the difference with its
+// partner and carry a rounding of the partner's size.  The z hops, which add the
+// neighbours' partners to every spin, bring one like it in either form;
+// norm-wise the errors agree (W^+W at 4^4 3.2e-16 and 3.4e-16).
 #include "kernels.cuh"
 #include "views.cuh"
 

@@ -362,9 +362,11 @@ __device__ __forceinline__ void clover_d_planes(L64& X, const Shifts& q, const d
 // 24^3x48: 1.30 ms for both parities and 0.73 ms for one, where the 20- to
 // 24-product form took 4.92 and 2.46 ms.  (The 8 link classes in sequence over
 // the lattice re-read the fields from HBM: 1.24 against 1.02 ms, averaged over
-// the two.)  Bound by FP64 arithmetic (51 products per link for both parities:
-// 0.78 ms at 18.9 T FMA/s) and the latency of its gathers.  2 CTAs per SM hold
-// X, k, t and a link without spilling; 3 spill 48 bytes and are no faster.
+// the two.)  Bound by FP64 arithmetic (per link and both parities 24 products
+// with a Hermitian matrix, 90 FMA each, and 25 others, 108 each: 0.68 ms at 18.9
+// T FMA/s, FP64 pipe 57 % busy) and by the latency of its gathers, 84 % of which
+// L2 serves.  2 CTAs per SM hold X, k, t and a link without spilling; 3 spill 48
+// bytes and are no faster.
 // eo_w 0, 1: w0 holds the planes of that parity; 2: w0 the even and w1 the
 // odd ones, both in one pass over the links
 __global__ void __launch_bounds__(kBlock, 2) k_clover_d(Geom g, double* p, const double2* gauge, const double* w0,
